@@ -35,12 +35,6 @@ namespace cfb {
 
 enum { MODEL_SUBSET = 0, MODEL_REPLACEMENT = 1 };
 
-#if defined(__CUDA_ARCH__)
-#define CF_LDG(p) __ldg(p)
-#else
-#define CF_LDG(p) (*(p))
-#endif
-
 // Scheduling controls for the hot loops.  Constant tables are interleaved (value, companion)
 // pairs fetched with one 16-byte load.  `ld_pair` is a volatile load and `pin` an empty volatile
 // statement that consumes a result: a load placed after a pin cannot be hoisted above the work
@@ -48,8 +42,11 @@ enum { MODEL_SUBSET = 0, MODEL_REPLACEMENT = 1 };
 //
 // L2 policy: the per-prime constant tables are re-read every step and are loaded with an
 // evict-last hint; the rows and column tiles of V and S stream through once per step and use
-// evict-first, so they do not push the tables out of L2.  V, S and the tiles are written by the
-// kernel itself, so they are read with plain coherent loads, never through the read-only path.
+// evict-first, so they do not push the tables out of L2.  Tables, V, S and the tiles are all written
+// by the kernel itself, so they are read with plain coherent loads, never through the read-only path
+// (ld.global.nc, __ldg): a read-only load is not ordered after the barrier that follows the write.
+// With read-only loads the 2^11 kernel at two CTAs per SM read table words of setup before they were
+// written (wrong residues on the first launch over a workspace).
 #if defined(__CUDA_ARCH__)
 CF_HD void pin(u64& v) { asm volatile("" : "+l"(v)); }
 CF_HD void pin_int(int& v) { asm volatile("" : "+r"(v)); }
@@ -64,7 +61,7 @@ CF_HD u64 policy_stream() {
     return pol;
 }
 CF_HD void ld_pair(const u64* p, u64& a, u64& b) {
-    asm volatile("ld.global.nc.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;" : "=l"(a), "=l"(b) : "l"(p), "l"(policy_keep()));
+    asm volatile("ld.global.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;" : "=l"(a), "=l"(b) : "l"(p), "l"(policy_keep()));
 }
 CF_HD u64 ld_stream(const u64* p) {
     u64 v;
@@ -89,10 +86,10 @@ CF_HD void pin(u64&) {}
 CF_HD void pin_int(int&) {}
 CF_HD void ld_pair(const u64* p, u64& a, u64& b) { a = p[0], b = p[1]; }
 #endif
-// Loads of data a kernel writes itself.  A CTA alone reads its own writes through L1 and the
-// read-only path.  In a cluster (CG), data another CTA wrote in this launch is read from L2 (.cg),
-// where the writer's release at the cluster barrier has made it visible; L1 lines of an earlier
-// read (block cells and tiles are reused) and the read-only path would not see the new values.
+// Loads of data a kernel writes itself.  A CTA alone reads its own writes through L1.  In a cluster
+// (CG), data another CTA wrote in this launch is read from L2 (.cg), where the writer's release at
+// the cluster barrier has made it visible; L1 lines of an earlier read (block cells and tiles are
+// reused) would not hold the new values.
 template <bool CG>
 CF_HD void ldp(const u64* p, u64& a, u64& b) {
 #if defined(__CUDA_ARCH__)
@@ -122,7 +119,7 @@ CF_HD u64 ldc(const u64* p) {
         u64 v;
         asm volatile("ld.global.cg.u64 %0, [%1];" : "=l"(v) : "l"(p));
         return v;
-    } else return CF_LDG(p);
+    } else return *p;
 #else
     return *p;
 #endif
