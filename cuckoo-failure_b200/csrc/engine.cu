@@ -17,8 +17,12 @@
 
 using namespace cfb;
 
-// The kernel for transform length 2^lg: primes below 2^50, or (wide) below 2^62.
-KInfo kernel_for(int lg, bool wide) {
+static int sm_count() {  // of the current device
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms;
+}
+KInfo kernel_for(int lg, bool wide, long primes) {
     if (wide) switch (lg) {
             case 4: return cf_kinfo_lg4_w();
             case 5: return cf_kinfo_lg5_w();
@@ -34,6 +38,12 @@ KInfo kernel_for(int lg, bool wide) {
             case 15: return cf_kinfo_lg15_c4_w();
             case 16: return cf_kinfo_lg16_c8_w();
             default: return KInfo{nullptr, 0, 0, 0};
+        }
+    if (few_per_sm(lg) > 0 && primes < MANY_PRIMES && primes <= (long)few_per_sm(lg) * sm_count()) switch (lg) {
+            case 8: return cf_kinfo_lg8_few();
+            case 9: return cf_kinfo_lg9_few();
+            case 10: return cf_kinfo_lg10_few();
+            case 12: return cf_kinfo_lg12_few();
         }
     switch (lg) {
         case 4: return cf_kinfo_lg4();
@@ -112,17 +122,18 @@ static int variants_for(int lg, KInfo* v, int cap) {
 }
 constexpr int MAX_VARIANTS = 8;
 // The kernel an engine runs: for primes below 2^50 the geometry it was tuned to, else the default.
-static KInfo kernel_of(const cf_engine* e, int lg, bool wide) {
+static KInfo kernel_of(const cf_engine* e, int lg, bool wide, long primes) {
     if (!wide && e && lg >= 0 && lg <= MAX_LG && e->tuned[lg] > 0) {
         KInfo v[MAX_VARIANTS];
         if (e->tuned[lg] < variants_for(lg, v, MAX_VARIANTS)) return v[e->tuned[lg]];
     }
-    return kernel_for(lg, wide);
+    return kernel_for(lg, wide, primes);
 }
 
 struct Plan {
     int lg, F, d0, nmax, J;
     bool wide = false;  // some prime is 2^50 or above: the kernels for primes below 2^62
+    long primes = MANY_PRIMES;  // primes of the batch, which its geometry follows
     KInfo ki;           // the kernel that runs the batch
     Layout lay;
     size_t ws_words;
@@ -130,7 +141,8 @@ struct Plan {
 // The kernel this engine runs for the plan and the workspace layout its geometry needs (the
 // pass-0 twiddle tables follow the entries per thread); again whenever wide or F changes.
 static int finalize(cf_engine* e, Plan& pl) {
-    pl.ki = kernel_of(e, pl.lg, pl.wide);
+    const long launch = e && e->max_ctas > 0 ? std::min<long>(pl.primes, e->max_ctas) : pl.primes;
+    pl.ki = kernel_of(e, pl.lg, pl.wide, launch);
     if (!pl.ki.fn) return fail(e, CF_ERR_UNSUPPORTED, "no kernel for this transform length");
     const int nw = pl.ki.threads >= 32 ? pl.ki.threads / 32 : 1;
     // cluster kernels: row sums for the largest cluster, so any cluster size can run the layout
@@ -168,6 +180,7 @@ static int plan(cf_engine* e, int nmax, int d, int model, const int* qn, const i
 static int check_primes(cf_engine* e, const u64* primes, int B, Plan& pl) {
     const u64 L = 1ull << pl.lg;
     pl.wide = false;
+    pl.primes = B;
     for (int b = 0; b < B; ++b) {
         const u64 p = primes[b];
         if (p < 3 || (p & 1) == 0 || p >= (1ull << 62) || p <= (u64)pl.F || (p - 1) % L != 0 || !cfh::is_prime(p))
@@ -642,6 +655,7 @@ int cf_residues_async(cf_engine* e, const uint64_t* d_primes, int B, int nmax, i
     if (rc) return rc;
     if (B == 0) return CF_OK;
     pl.wide = e->prime_bits > 50;
+    pl.primes = B;
     rc = finalize(e, pl);
     if (rc) return rc;
     CF_CUDA(cudaSetDevice(e->device), "set device");
@@ -723,6 +737,7 @@ int cf_batch_graph_create(cf_engine* e, const uint64_t* d_primes, int B, int nma
     int rc = plan(e, nmax, d, model, qn, qM, J, pl);
     if (rc) return rc;
     pl.wide = e->prime_bits > 50;
+    pl.primes = B;
     rc = finalize(e, pl);
     if (rc) return rc;
     CF_CUDA(cudaSetDevice(e->device), "set device");

@@ -3,3 +3,4 @@
 
 cfb::KInfo cf_kinfo_lg8() { return cfb::kinfo<8>(); }
 cfb::KInfo cf_kinfo_lg8_w() { return cfb::kinfo<8, true>(); }
+cfb::KInfo cf_kinfo_lg8_few() { return cfb::kinfo<8, false, true>(); }

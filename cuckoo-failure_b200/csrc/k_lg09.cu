@@ -3,3 +3,4 @@
 
 cfb::KInfo cf_kinfo_lg9() { return cfb::kinfo<9>(); }
 cfb::KInfo cf_kinfo_lg9_w() { return cfb::kinfo<9, true>(); }
+cfb::KInfo cf_kinfo_lg9_few() { return cfb::kinfo<9, false, true>(); }

@@ -3,3 +3,4 @@
 
 cfb::KInfo cf_kinfo_lg12() { return cfb::kinfo<12>(); }
 cfb::KInfo cf_kinfo_lg12_w() { return cfb::kinfo<12, true>(); }
+cfb::KInfo cf_kinfo_lg12_few() { return cfb::kinfo<12, false, true>(); }

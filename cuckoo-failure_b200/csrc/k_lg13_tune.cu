@@ -6,8 +6,8 @@ cfb::KInfo cf_kinfo_lg13();
 int cf_kvariants_lg13(cfb::KInfo* out, int cap) {
     const cfb::KInfo v[] = {
         cf_kinfo_lg13(),
-        cfb::kinfo_geo<13, 5, 1>(),
-        cfb::kinfo_geo<13, 4, 2>()};
+        cfb::kinfo_geo<13, 5, 2>(),
+        cfb::kinfo_geo<13, 3, 1>()};
     const int k = (int)(sizeof(v) / sizeof(v[0]));
     for (int i = 0; i < k && i < cap; ++i) out[i] = v[i];
     return k;

@@ -6,7 +6,7 @@ cfb::KInfo cf_kinfo_lg14();
 int cf_kvariants_lg14(cfb::KInfo* out, int cap) {
     const cfb::KInfo v[] = {
         cf_kinfo_lg14(),
-        cfb::kinfo_geo<14, 5, 1>()};
+        cfb::kinfo_geo<14, 4, 1>()};
     const int k = (int)(sizeof(v) / sizeof(v[0]));
     for (int i = 0; i < k && i < cap; ++i) out[i] = v[i];
     return k;

@@ -46,10 +46,10 @@ struct DevExec {
         asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ra), "l"(v) : "memory");
     }
     __device__ __forceinline__ void set_error(int* err, int code) { atomicCAS(err, 0, code); }
-    // Tensor memory: one warp allocates the CTA's columns (one CTA per SM uses it): all 512, or
-    // for a cluster's CTA the 4 E CT / 128 its threads use (a power of two, at least 32);
-    // thread t of warp w owns lane 32 (w % 4) + (t % 32), columns 4E (w / 4) + [0, 4E): E pairs.
-    static constexpr u32 TM_COLS = G::C == 1 ? 512 : (4 * G::E * (G::CT / 128) < 32 ? 32 : 4 * G::E * (G::CT / 128));
+    // Tensor memory: one warp allocates the columns the CTA's threads use, 4 E CT / 128 of the SM's
+    // 512 (a power of two, at least 32); thread t of warp w owns lane 32 (w % 4) + (t % 32), columns
+    // 4E (w / 4) + [0, 4E).
+    static constexpr u32 TM_COLS = 4 * G::E * (G::CT / 128) < 32 ? 32 : 4 * G::E * (G::CT / 128);
     static_assert((TM_COLS & (TM_COLS - 1)) == 0 && TM_COLS <= 512, "tensor memory columns: a power of two up to 512");
     __device__ __forceinline__ void tmem_alloc(u32* slot) {
         if ((threadIdx.x >> 5) == 0) {
@@ -114,17 +114,50 @@ struct DevExec {
     }
 };
 
-// Resident CTAs per SM the kernel is compiled for (registers per thread <= 65536 / (T x this)).
-// Measured on B200 (prime-residues/s, the same batch per SM, n = 2^LG):
-//   L = 2^10 (32 threads): 1 -> 6.9k, 12 -> 7.3k, 16 (128 registers, ptxas -O1) -> 8.9k: 16;
-//   L = 2^11 .. 2^13 (then with 32 entries per thread): capping registers lost 2 .. 20 %: 1 (no cap);
-//   L = 2^14: one CTA per SM is forced by its shared memory and tensor memory anyway.
-template <int LG>
-struct MinBlocks {
-    static constexpr int v = LG == 10 ? 16 : 1;
+// Default geometries by transform length 2^LG: 2^R entries per thread and MB resident CTAs per SM
+// (the register cap 65536 / (T MB)).
+//
+// Primes below 2^50 (double precision), measured on B200 (ms per launch, n = 2^LG or the stated n):
+//   2^14: 32 entries x 512 threads 703, 16 x 1024 853 (64 registers spill; n = 12500, 148 primes)
+//   2^13: 16 x 512, 128 registers 264; 32 x 256 371, 8 x 1024 297 (148 primes)
+//   2^12: 16 x 256 at 2 CTAs 238, 8 x 512 at 2 263, 32 x 128 at 4 329 (592 primes)
+//   2^11: 8 x 256 at 2 CTAs 132.5, at 4 (64 registers) 131, 16 x 128 at 4 139 (1184 primes)
+//   2^10: 8 x 128 at 4 CTAs 17.7, 4 x 256 at 2 21.1, at 4 19.6 (n = 1000, 592 primes)
+//   2^9:  8 x 64 at 8 CTAs 18.5, uncapped 23.2, 16 x 32 22.9 (2368 primes)
+//   2^8:  4 x 64 at 8 CTAs 5.6, uncapped 8.0, 8 x 32 6.7, 2 x 128 13.1 (2368 primes)
+//   2^7:  2 x 64 at 8 CTAs 1.80, 4 x 32 1.85 (n = 100, 2368 primes); 0.71 against 0.86 for 148 primes
+// FEW: for batches of few primes, which leave SMs with one or two CTAs, more threads per prime shorten
+// a step; used up to few_per_sm(LG) primes per SM:
+//   2^12: 8 x 512 at 148 primes 69.9 against 78.2, at 200 138.6 against 120.5 (n = 4096): 1 per SM
+//   2^10: 4 x 256 at 296 primes 10.6 against 12.0, at 444 18.1 against 14.5 (n = 1000): 2 per SM
+//   2^9:  4 x 128 at 148 primes 3.5 against 4.8, at 592 7.7 against 6.3: 2 per SM
+//   2^8:  2 x 128 at 148 primes 1.56 against 1.76, at 592 3.4 against 2.2: 1 per SM
+//
+// Primes below 2^62 (64-bit integers): 16 entries at 2^11 .. 2^14, 32 at 2^10 with 16 CTAs per SM.
+template <int LG, bool W, bool FEW = false>
+struct Geometry {
+    static constexpr int R = W          ? (LG >= 11 && LG <= 14 ? 4 : LG >= 10 ? 5 : LG >= 6 ? LG - 5 : 1)
+                             : LG == 14 ? 5
+                             : LG == 13 ? 4
+                             : LG == 12 ? (FEW ? 3 : 4)
+                             : LG == 11 ? 3
+                             : LG == 10 ? (FEW ? 2 : 3)
+                             : LG == 9  ? (FEW ? 2 : 3)
+                             : LG == 8  ? (FEW ? 1 : 2)
+                                        : 1;
+    static constexpr int MB = W          ? (LG == 10 ? 16 : 1)
+                              : LG >= 13 ? 1
+                              : LG == 12 ? (FEW ? 1 : 2)
+                              : LG == 11 ? 2
+                              : LG == 10 ? (FEW ? 2 : 4)
+                              : LG == 9  ? (FEW ? 1 : 8)
+                              : LG == 8  ? (FEW ? 1 : 8)
+                              : LG == 7  ? 8
+                                         : 1;
 };
+constexpr int few_per_sm(int lg) { return lg == 12 || lg == 8 ? 1 : lg == 10 || lg == 9 ? 2 : 0; }
 // MB: resident CTAs per SM the variant is compiled for (its register cap).
-template <int LG, int R, bool W, int MB = MinBlocks<LG>::v>
+template <int LG, int R, bool W, int MB>
 __global__ void __launch_bounds__(Geo<LG, R>::T, MB) k_suffix(KParams kp) {
     typedef Geo<LG, R> G;
     extern __shared__ __align__(16) u64 smem[];
@@ -151,8 +184,8 @@ struct QueueParams {
     const int* qM;
     const long long* qout;    // [sum J] output index of each query
 };
-template <int LG, int R, bool W>
-__global__ void __launch_bounds__(Geo<LG, R>::T, MinBlocks<LG>::v) k_suffix_queue(KParams kp, QueueParams qp) {
+template <int LG, int R, bool W, int MB>
+__global__ void __launch_bounds__(Geo<LG, R>::T, MB) k_suffix_queue(KParams kp, QueueParams qp) {
     typedef Geo<LG, R> G;
     typedef PrimeRun<G, DevExec<G>, W> PR;
     extern __shared__ __align__(16) u64 smem[];
@@ -160,7 +193,7 @@ __global__ void __launch_bounds__(Geo<LG, R>::T, MinBlocks<LG>::v) k_suffix_queu
     KParams& ikp = *reinterpret_cast<KParams*>(ikp_raw);
     __shared__ int item;
     DevExec<G> ex;
-    u32* tm_slot = (u32*)(smem + Smem<G>::MISC + MI_TMEM);
+    u32* tm_slot = (u32*)(smem + Smem<G, W>::MISC + MI_TMEM);
     if constexpr (PR::TM) ex.tmem_alloc(tm_slot);  // once for all the CTA's items
     for (;;) {
         if (threadIdx.x == 0) {
@@ -185,15 +218,6 @@ __global__ void __launch_bounds__(Geo<LG, R>::T, MinBlocks<LG>::v) k_suffix_queu
 }
 typedef void (*qfn_t)(KParams, QueueParams);
 
-// Elements per thread (2^R): 32 at L = 2^10, 16 at L = 2^11 .. 2^14, fewer below so a CTA keeps at
-// least a warp.  R = 4 was measured on B200 against R = 5 (twice the threads): n = 2048: 1826 ->
-// 2244, n = 4096: 496 -> 540, n = 8192: 122 -> 170, n = 16384: 40.8 -> 48.5 prime-residues/s
-// (1024 threads of 64 registers; 32 warps per SM hide the L2 latency of the per-step constants).
-template <int LG>
-struct RFor {
-    static constexpr int R = (LG >= 11 && LG <= 14) ? 4 : (LG >= 10 ? 5 : (LG >= 6 ? LG - 5 : 1));
-};
-
 typedef void (*kfn_t)(KParams);
 struct KInfo {
     kfn_t fn;
@@ -205,12 +229,12 @@ struct KInfo {
     int cluster = 1;  // CTAs per prime (a thread-block cluster when above 1)
     size_t smem_for(int J) const { return smem + (size_t)8 * J * (threads >= 32 ? threads / 32 : 1); }
 };
-// W selects the kernel for primes below 2^62 (otherwise below 2^50).
-template <int LG, bool W = false>
+// W selects the kernel for primes below 2^62 (otherwise below 2^50), FEW the geometry for few primes.
+template <int LG, bool W = false, bool FEW = false>
 inline KInfo kinfo() {
-    typedef Geo<LG, RFor<LG>::R> G;
-    return KInfo{&k_suffix<LG, RFor<LG>::R, W>, G::T, Smem<G>::BYTES, RFor<LG>::R, &k_suffix_queue<LG, RFor<LG>::R, W>,
-                 MinBlocks<LG>::v};
+    constexpr int R = Geometry<LG, W, FEW>::R, MB = Geometry<LG, W, FEW>::MB;
+    typedef Geo<LG, R> G;
+    return KInfo{&k_suffix<LG, R, W, MB>, G::T, Smem<G, W>::BYTES, R, &k_suffix_queue<LG, R, W, MB>, MB};
 }
 // Transform lengths above 2^14 (tables above n = 16384, primes below 2^50): one prime per cluster of
 // 2^LC CTAs, one CTA per SM, launched with that cluster size (CTA b 2^LC + c is CTA c of prime b).
@@ -227,13 +251,13 @@ __global__ void __launch_bounds__(Geo<LG, R, LC>::CT, 1) k_suffix_cl(KParams kp)
 template <int LG, int LC, int R = 4, bool W = false>
 inline KInfo kinfo_cluster() {
     typedef Geo<LG, R, LC> G;
-    return KInfo{&k_suffix_cl<LG, R, LC, W>, G::CT, Smem<G>::BYTES, R, nullptr, 1, G::C};
+    return KInfo{&k_suffix_cl<LG, R, LC, W>, G::CT, Smem<G, W>::BYTES, R, nullptr, 1, G::C};
 }
 // Another geometry of the 50-bit kernel (autotuning candidates): 2^R entries per thread, MB CTAs per SM.
 template <int LG, int R, int MB>
 inline KInfo kinfo_geo() {
     typedef Geo<LG, R> G;
-    return KInfo{&k_suffix<LG, R, false, MB>, G::T, Smem<G>::BYTES, R, nullptr, MB};
+    return KInfo{&k_suffix<LG, R, false, MB>, G::T, Smem<G, 0>::BYTES, R, nullptr, MB};
 }
 
 }  // namespace cfb

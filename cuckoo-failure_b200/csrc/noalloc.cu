@@ -26,32 +26,9 @@
 
 #include "../../include/cuckoo_b200.h"
 #include "host_common.hpp"
-#include "kernel_lg.cuh"
+#include "engine_internal.hpp"
 
 using namespace cfb;
-
-cfb::KInfo cf_kinfo_lg4();
-cfb::KInfo cf_kinfo_lg5();
-cfb::KInfo cf_kinfo_lg6();
-cfb::KInfo cf_kinfo_lg7();
-cfb::KInfo cf_kinfo_lg8();
-cfb::KInfo cf_kinfo_lg9();
-cfb::KInfo cf_kinfo_lg10();
-cfb::KInfo cf_kinfo_lg11();
-cfb::KInfo cf_kinfo_lg12();
-cfb::KInfo cf_kinfo_lg13();
-cfb::KInfo cf_kinfo_lg14();
-cfb::KInfo cf_kinfo_lg4_w();
-cfb::KInfo cf_kinfo_lg5_w();
-cfb::KInfo cf_kinfo_lg6_w();
-cfb::KInfo cf_kinfo_lg7_w();
-cfb::KInfo cf_kinfo_lg8_w();
-cfb::KInfo cf_kinfo_lg9_w();
-cfb::KInfo cf_kinfo_lg10_w();
-cfb::KInfo cf_kinfo_lg11_w();
-cfb::KInfo cf_kinfo_lg12_w();
-cfb::KInfo cf_kinfo_lg13_w();
-cfb::KInfo cf_kinfo_lg14_w();
 
 namespace {
 
@@ -66,38 +43,6 @@ __device__ __align__(256) u64 g_noalloc_scratch[SCRATCH_WORDS];
 std::mutex g_mu;
 u64* g_scratch_ptr[MAX_DEVICES] = {};
 std::string g_err;
-
-// wide: some prime is 2^50 or above (the kernels for primes below 2^62)
-KInfo kernel_for(int lg, bool wide) {
-    if (wide) switch (lg) {
-            case 4: return cf_kinfo_lg4_w();
-            case 5: return cf_kinfo_lg5_w();
-            case 6: return cf_kinfo_lg6_w();
-            case 7: return cf_kinfo_lg7_w();
-            case 8: return cf_kinfo_lg8_w();
-            case 9: return cf_kinfo_lg9_w();
-            case 10: return cf_kinfo_lg10_w();
-            case 11: return cf_kinfo_lg11_w();
-            case 12: return cf_kinfo_lg12_w();
-            case 13: return cf_kinfo_lg13_w();
-            case 14: return cf_kinfo_lg14_w();
-            default: return KInfo{nullptr, 0, 0, 0};
-        }
-    switch (lg) {
-        case 4: return cf_kinfo_lg4();
-        case 5: return cf_kinfo_lg5();
-        case 6: return cf_kinfo_lg6();
-        case 7: return cf_kinfo_lg7();
-        case 8: return cf_kinfo_lg8();
-        case 9: return cf_kinfo_lg9();
-        case 10: return cf_kinfo_lg10();
-        case 11: return cf_kinfo_lg11();
-        case 12: return cf_kinfo_lg12();
-        case 13: return cf_kinfo_lg13();
-        case 14: return cf_kinfo_lg14();
-        default: return KInfo{nullptr, 0, 0, 0};
-    }
-}
 
 int fail(int code, const std::string& msg) {
     g_err = msg;
@@ -148,7 +93,7 @@ extern "C" int cf_residues_noalloc(const uint64_t* primes, int B, int nmax, int 
             return fail(CF_ERR_ARG, "prime " + std::to_string(p) + " is not an odd prime < 2^62 above max(n, M) with L | p-1");
         if (p >= (1ull << 50)) wide = true;
     }
-    const KInfo ki = kernel_for(lg, wide);
+    const KInfo ki = kernel_for(lg, wide, B);
     if (!ki.fn) return fail(CF_ERR_UNSUPPORTED, "no kernel for this transform length");
     if (B == 0) return CF_OK;
     const Layout lay = make_layout(nmax, F, (int)L, J, ki.threads >= 32 ? ki.threads / 32 : 1, ki.r);

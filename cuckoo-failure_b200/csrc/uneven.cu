@@ -147,7 +147,7 @@ int cf_uneven_create(cf_engine* e, const int* n, const int* M, const int* d, int
                 ++b;
             }
             g.b = b;
-            g.ki = kernel_for(g.lg, wide);
+            g.ki = kernel_for(g.lg, wide, (long)(b - a));
             if (!g.ki.qfn) return fail(e, CF_ERR_UNSUPPORTED, "no kernel for this transform length");
             const int nw = g.ki.threads >= 32 ? g.ki.threads / 32 : 1;
             g.lay = make_layout(g.nmax, g.F, 1 << g.lg, g.J, nw, g.ki.r);
