@@ -534,21 +534,30 @@ static int tables_query(cf_engine* e, const cf_tables* t, const int* qn, const i
             return fail(e, CF_ERR_ARG, "query needs 1 <= n <= table n and n < M <= table F");
         if (t->model == CF_MODEL_SUBSET && t->d > qM[j]) return fail(e, CF_ERR_ARG, "subset model needs d <= M");
     }
-    const size_t smem = tq_smem_bytes(t->n);
-    CF_CUDA(cudaFuncSetAttribute((const void*)k_table_query<TQ_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-            "shared memory attribute");
+    const int sms = sm_count();
+    std::vector<int> order;
     for (int j0 = 0; j0 < J; j0 += TQ_MAXJ) {
         TQParams tp;
         tp.primes = t->d_primes;
         tp.B = t->B, tp.n = t->n, tp.F = t->F, tp.d = t->d, tp.d0 = t->d0, tp.model = t->model;
         tp.J = std::min(TQ_MAXJ, J - j0);
-        for (int j = 0; j < tp.J; ++j) tp.qn[j] = qn[j0 + j], tp.qM[j] = qM[j0 + j];
+        order.resize((size_t)tp.J);
+        for (int j = 0; j < tp.J; ++j) order[(size_t)j] = j0 + j;
+        std::sort(order.begin(), order.end(), [&](int a, int b) { return qn[a] > qn[b]; });  // largest tables first
+        for (int j = 0; j < tp.J; ++j) tp.qn[j] = qn[order[(size_t)j]], tp.qM[j] = qM[order[(size_t)j]], tp.qi[j] = (short)(order[(size_t)j] - j0);
         tp.keep = t->keep;
         tp.keep_words = t->keep_words;
         tp.out = d_out + j0;
         tp.out_stride = (size_t)J;
-        k_table_query<TQ_THREADS><<<t->B * tp.J, TQ_THREADS, smem, s>>>(tp);
-        CF_CUDA(cudaGetLastError(), "query launch");
+        tp.S = tq_ctas(t->B, tp.qn[0], sms);
+        const size_t smem = tq_smem_bytes(tp.J);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute att[1];
+        att[0].id = cudaLaunchAttributeClusterDimension;
+        att[0].val.clusterDim.x = (unsigned)tp.S, att[0].val.clusterDim.y = 1, att[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(t->B * tp.S)), cfg.blockDim = dim3(TQ_THREADS), cfg.dynamicSmemBytes = smem;
+        cfg.stream = s, cfg.attrs = att, cfg.numAttrs = 1;
+        CF_CUDA(cudaLaunchKernelEx(&cfg, k_table_query, tp), "query launch");
         ++e->launches;
     }
     return CF_OK;

@@ -1,9 +1,20 @@
 // Queries served from resident tables (cf_tables_query): N_bad(n, M) mod p for primes whose whole
-// V (packed triangle) and pair tables fact, ifact, inv were kept by a serving build
-// (KParams::keep).  The arithmetic is that of the build's own query and finish phases
-// (PrimeRun::query_row and PrimeRun::finish): the per-row sums of fast/cuckoo_fast.cu:306-323,
-// 595-622 and the Horner finish of :877-890, read from the resident triangle instead of from the
-// row the build is about to consume.
+// V (packed triangle) and tables fact, ifact, inv were kept by a serving build (KParams::keep).  The
+// arithmetic is that of the build's own query and finish phases (query_row and finish in
+// prime_fp.cuh): the per-row sums of fast/cuckoo_fast.cu:306-323, 595-622 and the Horner finish of
+// :877-890, read from the resident triangle instead of from the row the build is about to consume.
+//
+// The rows' factors F(q) = inv[q] ifact[n-q] ifact[M-q] Q^(n-q) go in front of the inner sums:
+//   sum_q F(q) sum_w Vs[q][w] / (M-w)  =  sum_w 1/(M-w) sum_q F(q) Vs[q][w],
+// so a warp takes TQ_ROWS rows of TQ_COLS columns, each lane its own columns down the rows: an entry
+// costs one product by a factor all lanes share, the inverses enter once per column, and nothing is
+// summed across lanes but the tile's total.  A prime's tiles go to the warps of a cluster of CTAs.
+//
+// Bound by the triangle's bytes where few queries read it (8 queries, two of them as large as the
+// table, n = 2048, 148 primes: 2.5 GB), by the products (seven double-precision operations each) where
+// many do.  A warp reads 2 KB of a row at a time, a row ahead: with 256 bytes of four rows at a
+// time, summing along the rows, HBM gave 2.2 TB/s (1320 us for that case); the form before that, one
+// CTA of 64-bit integer products per (prime, query), took 3570 us; this one takes 610 (4.1 TB/s).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -16,86 +27,168 @@ namespace cfb {
 constexpr int TQ_MAXJ = 256;
 struct TQParams {
     const u64* primes;  // [B]
-    int B, n, F, d, d0, model, J;
+    int B, n, F, d, d0, model, J, S;  // S: CTAs per prime
     const u64* keep;    // [B][keep_words]
     size_t keep_words;
     u64* out;           // residue of prime b, query jq at out[b * out_stride + jq]
     size_t out_stride;
-    int qn[TQ_MAXJ];    // each <= n
+    int qn[TQ_MAXJ];    // each <= n, descending
     int qM[TQ_MAXJ];    // each <= F
+    short qi[TQ_MAXJ];  // the query's place in out
 };
 
-// One CTA per (prime, query).  Dynamic shared memory: the row sums ps[0..n] and a reduction area.
-template <int T>
-__global__ void __launch_bounds__(T) k_table_query(TQParams tp) {
-    constexpr int NW = T / 32;
-    extern __shared__ __align__(16) u64 sq[];
-    const int b = blockIdx.x / tp.J, jq = blockIdx.x % tp.J;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int nj = tp.qn[jq], Mj = tp.qM[jq], d0 = tp.d0;
-    u64* ps = sq;             // [n + 1] row sums
-    u64* red = sq + tp.n + 1;  // [NW + 1]
-    __shared__ Mod smod;
-    __shared__ u64 soneq;
-    const u64 P = tp.primes[b];
-    if (t == 0) {
-        smod = make_mod(P);
-        soneq = shoup_companion(1, P);
-    }
-    const KeepLayout kl = make_keep_layout(tp.n, tp.F);
-    const u64* base = tp.keep + (size_t)b * tp.keep_words;
-    const u64* tri = base + kl.tri;
-    const u64* fact = base + kl.fact;
-    const u64* ifact = base + kl.ifact;
-    const u64* inv = base + kl.inv;
-    auto sh = [&](u64 a, const u64* pairs, int k) { return shoup_mul_lazy(a, pairs[2 * k], pairs[2 * k + 1], P); };
-    for (int q = t; q <= nj; q += T) ps[q] = 0;
-    __syncthreads();
-    const u64 oneq = soneq;
-    // ps[q] = sum_{d0 <= w < q} Vs[q][w] / (M - w): one warp per row, lanes along the row
-    for (int q = d0 + 1 + warp; q <= nj; q += NW) {
-        const u64* row = tri + tri_off(q);
-        u64 acc = 0;  // each term < 4p < 2^52, at most 512 terms per lane
-        for (int w = d0 + lane; w < q; w += 32) acc += sh(row[w], inv, Mj - w);
-        u64 v = shoup_mul_lazy(acc, 1, oneq, P);
-        v = v >= 2 * P ? v - 2 * P : v;
-        v = v >= P ? v - P : v;
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) v = madd(v, __shfl_xor_sync(0xffffffffu, v, o), P);
-        if (lane == 0) ps[q] = v;
-    }
-    __syncthreads();
-    // N_bad = M! n! sum_k inv[k] ifact[n-k] ifact[M-k] Q^(n-k) ps[k]
-    const Mod m = smod;
-    u64 Qm;
-    if (tp.model == MODEL_REPLACEMENT) Qm = mont_pow(to_mont((u64)Mj, m), (u64)tp.d, m);
-    else {
-        const u64 c = sh(sh(fact[2 * Mj], ifact, tp.d), ifact, Mj - tp.d);
-        Qm = to_mont(red2(red2(c, 2 * P), P), m);
-    }
-    u64 acc = 0;
-    for (int k = t + 1; k <= nj; k += T) {
-        u64 y = sh(ps[k], inv, k);
-        y = sh(y, ifact, nj - k);
-        y = sh(y, ifact, Mj - k);
-        y = mont_mul(y, mont_pow(Qm, (u64)(nj - k), m), m);
-        acc = madd(acc, y, P);
-    }
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) acc = madd(acc, __shfl_xor_sync(0xffffffffu, acc, o), P);
-    if (lane == 0) red[warp] = acc;
-    __syncthreads();
-    if (t == 0) {
-        u64 s = 0;
-        for (int w = 0; w < NW; ++w) s = madd(s, red[w], P);
-        u64 r = sh(s, fact, nj);
-        r = red2(red2(r, 2 * P), P);
-        r = sh(r, fact, Mj);
-        tp.out[(size_t)b * tp.out_stride + jq] = red2(red2(r, 2 * P), P);
-    }
+constexpr int TQ_THREADS = 256, TQ_WARPS = TQ_THREADS / 32, TQ_PER_SM = 2;
+constexpr int TQ_ROWS = 16, TQ_K = 8, TQ_COLS = 32 * TQ_K;  // a warp's tile: rows, columns per lane, columns
+constexpr int TQ_CLUSTER = 8;                               // CTAs per prime at most
+// Shared memory: per query Q and the warps' sums, and (read from the first CTA) the CTAs' sums.
+inline size_t tq_smem_bytes(int J) { return 8 * (size_t)J * (1 + TQ_WARPS + TQ_CLUSTER); }
+// CTAs per prime: the number up to TQ_CLUSTER whose waves of resident CTAs leave the least idle (the
+// CTAs' shares are equal, so a launch lasts waves / S), with a block of rows for every warp.
+inline int tq_ctas(int B, int nmax, int sms) {
+    const long cap = (long)TQ_PER_SM * (sms > 0 ? sms : 1);
+    int S = 1;
+    for (int c = 2; c <= TQ_CLUSTER && nmax >= TQ_ROWS * TQ_WARPS * c / 2; ++c)
+        if (((long)B * c + cap - 1) / cap * S < ((long)B * S + cap - 1) / cap * c) S = c;
+    return S;
 }
 
-constexpr int TQ_THREADS = 256;
-inline size_t tq_smem_bytes(int n) { return 8 * ((size_t)n + 1 + TQ_THREADS / 32 + 1); }
+// a whole number below 2^52 as a double
+__device__ __forceinline__ double tq_double(u64 v) { return __dadd_rn(__longlong_as_double((long long)(v | 0x4330000000000000ull)), -4503599627370496.0); }
+__device__ __forceinline__ double tq_load(const u64* p) { return tq_double(__ldg(p)); }  // resident tables: another launch's writes
+
+// One tile, rows q0 .. q0 + TQ_ROWS - 1 and columns w0 .. w0 + TQ_COLS - 1, for queries j0 .. j0 + NJ - 1:
+// its part of their sums is added to sums[].
+template <int NJ>
+__device__ __forceinline__ void tq_tile(const TQParams& tp, const KeepLayout& kl, const u64* base, const FpMod& m, int q0, int w0,
+                                        int j0, const double* Qs, double* sums) {
+    const int lane = threadIdx.x & 31, d0 = tp.d0;
+    const u64* inv = base + kl.inv;
+    const u64* tri = base + kl.tri + w0 + lane;
+    const int qe = min(q0 + TQ_ROWS - 1, tp.qn[j0]);  // the last row a query needs (sizes descend)
+    u64 next[TQ_K];
+    auto get = [&](int q) {
+        const u64* row = tri + tri_off((size_t)q);
+#pragma unroll
+        for (int k = 0; k < TQ_K; ++k) {
+            const int w = w0 + lane + 32 * k;
+            next[k] = w < q && w >= d0 && q <= qe ? __ldg(row + 32 * k) : 0;  // resident tables: another launch's writes
+        }
+    };
+    get(q0);
+    // lane r + TQ_ROWS j computes F of row q0 + r for query j0 + j (zero past the query's size)
+    double F = 0;
+    {
+        const int j = NJ > 1 ? j0 + lane / TQ_ROWS : j0, q = q0 + lane % TQ_ROWS, nj = tp.qn[j], Mj = tp.qM[j];
+        if (q <= nj) {
+            F = fp_mulmod(tq_load(inv + 2 * (size_t)q), tq_load(base + kl.ifact + 2 * (size_t)(nj - q)), m);
+            F = fp_mulmod(F, tq_load(base + kl.ifact + 2 * (size_t)(Mj - q)), m);
+            F = fp_mulmod(F, fp_pow(Qs[j], (u64)(nj - q), m), m);
+        }
+    }
+    double acc[NJ][TQ_K];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int k = 0; k < TQ_K; ++k) acc[j][k] = 0;
+#pragma unroll 1
+    for (int r = 0; r < TQ_ROWS && q0 + r <= qe; ++r) {
+        double x[TQ_K];
+#pragma unroll
+        for (int k = 0; k < TQ_K; ++k) x[k] = tq_double(next[k]);
+        get(q0 + r + 1);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const double f = __shfl_sync(0xffffffffu, F, r + TQ_ROWS * j);
+#pragma unroll
+            for (int k = 0; k < TQ_K; ++k) acc[j][k] = fp_add(acc[j][k], fp_mulmod(x[k], f, m));
+        }
+        if ((r & 7) == 7)  // at most eight terms below 0.67p and the sum below 0.51p
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                for (int k = 0; k < TQ_K; ++k) acc[j][k] = fp_red(acc[j][k], m);
+    }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+        const int Mj = tp.qM[j0 + j];
+        double y = 0;
+#pragma unroll
+        for (int k = 0; k < TQ_K; ++k) {
+            const int w = w0 + lane + 32 * k;  // columns at or past the query's size hold zero
+            const double c = w < qe && w < Mj ? tq_load(inv + 2 * (size_t)(Mj - w)) : 0.0;
+            y = fp_add(y, fp_mulmod(fp_red(acc[j][k], m), c, m));  // eight below 0.65p
+        }
+        y = fp_red(y, m);
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) {
+            y = fp_add(y, __shfl_xor_sync(0xffffffffu, y, o));
+            if (o == 4) y = fp_red(y, m);
+        }
+        if (lane == 0) sums[j0 + j] = fp_red(fp_add(sums[j0 + j], y), m);
+    }
+    __syncwarp();
+}
+
+// S CTAs (a cluster) per prime: CTA b S + s is CTA s of prime b.
+__global__ void __launch_bounds__(TQ_THREADS, TQ_PER_SM) k_table_query(TQParams tp) {
+    extern __shared__ __align__(16) double tq_sm[];
+    const int S = tp.S, b = blockIdx.x / S, s = blockIdx.x % S, J = tp.J;
+    const int t = threadIdx.x, warp = t >> 5;
+    double* Qs = tq_sm;                    // [J] candidate sets per item
+    double* sums = tq_sm + J;              // [TQ_WARPS][J]
+    double* all = sums + TQ_WARPS * J;     // [S][J], in the cluster's first CTA
+    const u64 P = tp.primes[b];
+    FpMod m;
+    m.p = tq_double(P), m.pinv = 1.0 / m.p;
+    const KeepLayout kl = make_keep_layout(tp.n, tp.F);
+    const u64* base = tp.keep + (size_t)b * tp.keep_words;
+    const u64 *fact = base + kl.fact, *ifact = base + kl.ifact;
+    for (int j = t; j < J; j += TQ_THREADS) {
+        const int Mj = tp.qM[j];
+        Qs[j] = tp.model == MODEL_REPLACEMENT
+                    ? fp_pow((double)Mj, (u64)tp.d, m)
+                    : fp_mulmod(fp_mulmod(tq_load(fact + 2 * (size_t)Mj), tq_load(ifact + 2 * (size_t)tp.d), m), tq_load(ifact + 2 * (size_t)(Mj - tp.d)), m);
+    }
+    for (int k = t; k < TQ_WARPS * J; k += TQ_THREADS) sums[k] = 0;
+    __syncthreads();
+    // tiles, the last rows first, dealt to the prime's warps in turn
+    const int nw = S * TQ_WARPS, me = warp * S + s;
+    int at = 0;
+    for (int blk = (tp.qn[0] - 1) / TQ_ROWS; blk >= 0; --blk) {
+        const int q0 = 1 + TQ_ROWS * blk, tiles = (min(q0 + TQ_ROWS - 1, tp.qn[0]) + TQ_COLS - 1) / TQ_COLS;  // columns 0 .. q0 + TQ_ROWS - 2
+        if (q0 + TQ_ROWS - 1 <= tp.d0) break;
+        for (int c = (me - at % nw + nw) % nw; c < tiles; c += nw)
+            for (int j = 0; j < J && tp.qn[j] >= q0;) {
+                if (j + 1 < J && tp.qn[j + 1] >= q0) tq_tile<2>(tp, kl, base, m, q0, c * TQ_COLS, j, Qs, sums + warp * J), j += 2;
+                else tq_tile<1>(tp, kl, base, m, q0, c * TQ_COLS, j, Qs, sums + warp * J), j += 1;
+            }
+        at += tiles;
+    }
+    __syncthreads();
+    for (int j = t; j < J; j += TQ_THREADS) {
+        double a = 0;
+        for (int w = 0; w < TQ_WARPS; ++w) a = fp_add(a, sums[w * J + j]);  // eight below 0.51p
+        a = fp_red(a, m);
+        if (S == 1) all[j] = a;
+        else {
+            u32 ra;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"((u32)__cvta_generic_to_shared(all + s * J + j)), "r"(0));
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(a) : "memory");
+        }
+    }
+    if (S == 1) __syncthreads();
+    else {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    if (s) return;
+    for (int j = t; j < J; j += TQ_THREADS) {  // N_bad = M! n! sum of the terms
+        double a = 0;
+        for (int c = 0; c < S; ++c) a = fp_add(a, all[c * J + j]);
+        a = fp_mulmod(fp_red(a, m), tq_load(fact + 2 * (size_t)tp.qn[j]), m);
+        a = fp_mulmod(a, tq_load(fact + 2 * (size_t)tp.qM[j]), m);
+        tp.out[(size_t)b * tp.out_stride + tp.qi[j]] = fp_canon(a, m);
+    }
+}
 
 }  // namespace cfb
