@@ -226,15 +226,33 @@ static long fit_batch(size_t per_prime) {
     return (long)((fr - reserve) / per_prime);
 }
 
-// A launch keeps the per-warp partial sums of its J queries in shared memory (8 J words per warp)
-// beside the kernel's fixed part; more queries than the block's opt-in limit allows are refused.
-int check_smem(cf_engine* e, size_t smem, int J) {
+// Queries a launch takes at transform length 2^lg: what fits a block's shared memory (optin bytes) beside
+// the exchange area when every warp of a geometry of 16 entries per thread (32 at 2^10, two or more
+// below, at least a warp) keeps a partial sum per query.  Kernels with more warps sum them in batches.
+int query_cap(int lg, const KInfo& ki, int optin) {
+    const long L = 1l << lg;
+    long words, nw;
+    if (ki.cluster > 1) {
+        const long ct = ki.threads;
+        words = 2 * L / ki.cluster + 2 * ct + 64 + 16 + 2 * ((L >> (ki.r + 1)) + 1) + 208, nw = ct / 32;
+        words = std::max(words, 120l * 128);
+    } else {
+        const int r = lg >= 11 ? 4 : lg >= 10 ? 5 : lg >= 6 ? lg - 5 : 1;
+        const long t = L >> r;
+        words = L + 2 * t + 64 + 16 + 2 * ((L >> (r + 1)) + 1) + 208, nw = std::max(1l, t / 32);
+    }
+    return (int)std::max(0l, (optin - 8 * words) / (8 * nw));
+}
+int plan_queries(cf_engine* e, int lg, const KInfo& ki, int J, size_t* smem, int* JC) {
     int dev = 0, optin = 0;
     CF_CUDA(cudaGetDevice(&dev), "current device");
     CF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "shared memory limit");
-    if (smem > (size_t)optin)
-        return fail(e, CF_ERR_UNSUPPORTED, std::to_string(J) + " queries need " + std::to_string(smem) +
-                                               " bytes of shared memory per block; the device allows " + std::to_string(optin));
+    const int cap = query_cap(lg, ki, optin);
+    if (J > cap)
+        return fail(e, CF_ERR_UNSUPPORTED, std::to_string(J) + " queries need more shared memory per block than the device allows (" +
+                                               std::to_string(optin) + " bytes, " + std::to_string(cap) + " queries)");
+    *JC = ki.batch_for(J, optin);
+    *smem = ki.smem_for(*JC);
     return CF_OK;
 }
 
@@ -247,9 +265,10 @@ static int launch_batch(cf_engine* e, const u64* d_primes, int B, int nmax, int 
     KInfo ki = pl.ki;
     if (!ki.fn) return fail(e, CF_ERR_UNSUPPORTED, "no kernel for this transform length");
     if (ki.cluster > 1 && keep) return fail(e, CF_ERR_UNSUPPORTED, "resident tables are built up to nmax = 16384");
-    if (ki.cluster > 1) ki = pick_cluster(e, pl.lg, B, J, s, pl.wide);  // refined per chunk below
-    size_t smem = ki.smem_for(J);
-    int rc0 = check_smem(e, smem, J);
+    if (ki.cluster > 1) ki = pick_cluster(e, pl.lg, B, J, s, pl.wide);
+    size_t smem = 0;
+    int JC = 0;
+    int rc0 = plan_queries(e, pl.lg, ki, J, &smem, &JC);
     if (rc0) return rc0;
     CF_CUDA(cudaFuncSetAttribute((const void*)ki.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
             "shared memory attribute");
@@ -292,11 +311,8 @@ static int launch_batch(cf_engine* e, const u64* d_primes, int B, int nmax, int 
         kp.err = err;
         kp.keep = keep ? keep + (size_t)at * keep_words : nullptr;
         kp.keep_words = keep_words;
+        kp.JC = JC;
         if (ki.cluster > 1) {  // one cluster of ki.cluster CTAs per prime
-            ki = pick_cluster(e, pl.lg, nb, J, s, pl.wide);
-            smem = ki.smem_for(J);
-            rc0 = check_smem(e, smem, J);
-            if (rc0) return rc0;
             CF_CUDA(cudaFuncSetAttribute((const void*)ki.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                     "shared memory attribute");
             if (ki.cluster > 8)
@@ -629,7 +645,9 @@ long cf_resident_primes(cf_engine* e, int nmax, int Mmax, int J) {
     Plan pl;
     if (plan(e, nmax, 3, CF_MODEL_SUBSET, qn.data(), qM.data(), J, pl)) return 0;
     const KInfo ki = pl.ki.cluster > 1 ? pick_cluster(e, pl.lg, 1, J, e->stream) : pl.ki;
-    const size_t smem = ki.smem_for(J);
+    size_t smem = 0;
+    int JC = 0;
+    if (plan_queries(e, pl.lg, ki, J, &smem, &JC)) return 0;
     if (ki.cluster > 1) return resident_clusters(ki, smem, e->stream);
     int per_sm = 0, sms = 0;
     if (cudaFuncSetAttribute((const void*)ki.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||

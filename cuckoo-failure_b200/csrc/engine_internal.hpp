@@ -53,8 +53,10 @@ constexpr int MAX_LG = 14;          // one CTA per prime (every entry point)
 constexpr int MAX_LG_CLUSTER = 16;  // a cluster of CTAs per prime (cf_residues and its forms)
 constexpr int MAX_CLUSTER = 16;     // the largest cluster a layout provides row sums for
 struct cf_engine;
-// CF_OK if a launch with J queries fits the device's shared memory per block (engine.cu)
-int check_smem(cf_engine* e, size_t smem, int J);
+// The shared memory of a launch of ki with J queries at transform length 2^lg, and how many of them it
+// sums at a time; CF_ERR_UNSUPPORTED above the queries a launch takes (engine.cu).
+int plan_queries(cf_engine* e, int lg, const cfb::KInfo& ki, int J, size_t* smem, int* JC);
+int query_cap(int lg, const cfb::KInfo& ki, int optin);
 
 // ------------------------------------------------------------------------------------------
 // Engine

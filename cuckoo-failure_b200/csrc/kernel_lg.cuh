@@ -133,10 +133,15 @@ struct DevExec {
 //   2^9:  4 x 128 at 148 primes 3.5 against 4.8, at 592 7.7 against 6.3: 2 per SM
 //   2^8:  2 x 128 at 148 primes 1.56 against 1.76, at 592 3.4 against 2.2: 1 per SM
 //
-// Primes below 2^62 (64-bit integers): 16 entries at 2^11 .. 2^14, 32 at 2^10 with 16 CTAs per SM.
+// Primes below 2^62 (64-bit integers), one CTA's registers uncapped (ms per launch, n = 2^LG or the
+// stated n; in front the geometries with half to an eighth of the threads that were the default):
+//   2^13: 16 x 512 941, 8 x 1024 762 (148 primes)     2^12: 16 x 256 269, 8 x 512 179, 4 x 1024 200 (148)
+//   2^11: 16 x 128 126, 8 x 256 72, 4 x 512 51 (148); 271, 288, 204 (592)
+//   2^10: 32 x 32 126, 8 x 128 32, 4 x 256 14.4 (n = 1000, 148); 499, 270, 229 (2368)
+//   2^9:  16 x 32 30, 4 x 128 6.2, 2 x 256 5.5 (148); 34, 17, 21 (592)   2^8: 8 x 32 7.2, 4 x 64 2.9 (148); 8.1, 3.8 (592)
 template <int LG, bool W, bool FEW = false>
 struct Geometry {
-    static constexpr int R = W          ? (LG >= 11 && LG <= 14 ? 4 : LG >= 10 ? 5 : LG >= 6 ? LG - 5 : 1)
+    static constexpr int R = W          ? (LG == 14 ? 4 : LG >= 12 ? 3 : LG >= 10 ? 2 : LG >= 8 ? 2 : 1)
                              : LG == 14 ? 5
                              : LG == 13 ? 4
                              : LG == 12 ? (FEW ? 3 : 4)
@@ -145,7 +150,7 @@ struct Geometry {
                              : LG == 9  ? (FEW ? 2 : 3)
                              : LG == 8  ? (FEW ? 1 : 2)
                                         : 1;
-    static constexpr int MB = W          ? (LG == 10 ? 16 : 1)
+    static constexpr int MB = W          ? 1
                               : LG >= 13 ? 1
                               : LG == 12 ? (FEW ? 1 : 2)
                               : LG == 11 ? 2
@@ -222,12 +227,18 @@ typedef void (*kfn_t)(KParams);
 struct KInfo {
     kfn_t fn;
     int threads;  // per CTA
-    size_t smem;  // fixed dynamic shared memory; a launch with J queries adds 8 J (threads / 32)
+    size_t smem;  // fixed dynamic shared memory; JC queries at a time add 8 JC (threads / 32)
     int r;        // log2 of the entries per thread
     qfn_t qfn;    // the work-queue form (the default geometry only)
     int mb;       // resident CTAs per SM the kernel is compiled for
     int cluster = 1;  // CTAs per prime (a thread-block cluster when above 1)
-    size_t smem_for(int J) const { return smem + (size_t)8 * J * (threads >= 32 ? threads / 32 : 1); }
+    int warps() const { return threads >= 32 ? threads / 32 : 1; }
+    size_t smem_for(int JC) const { return smem + (size_t)8 * JC * warps(); }
+    // queries whose partial sums a block's shared memory (optin bytes) holds at a time, at most J
+    int batch_for(int J, int optin) const {
+        const long fit = (long)optin > (long)smem ? ((long)optin - (long)smem) / (8 * warps()) : 0;
+        return (int)(fit < J ? (fit > 0 ? fit : 1) : J);
+    }
 };
 // W selects the kernel for primes below 2^62 (otherwise below 2^50), FEW the geometry for few primes.
 template <int LG, bool W = false, bool FEW = false>

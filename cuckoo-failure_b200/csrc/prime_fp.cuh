@@ -85,7 +85,7 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
     using Base::md;
     using Base::sum_red;
     typedef typename Base::Row Row;
-    using Base::fold_queries;
+    using Base::fold_last;
     typedef Bounds<G> BD;
     static constexpr int R = G::R, LG = G::LG, RL = G::R_LAST;
 
@@ -322,7 +322,7 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
     // Work done behind a convolution's first barrier, where the groups of threads go on alone, so the
     // few warps that do it delay nobody: row fold_'s query partials, the power tables of step pow_.
     CF_HD void chain_work() {
-        if (fold_) fold_queries(fold_);
+        if (fold_) fold_last(fold_);
         if (pow_) ex.each([&](int t, Regs<G>&) CF_INL { power_tables(t, pow_); });
     }
     template <int PASS>
@@ -707,14 +707,12 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
     // (the U[w] / (M - w) sums of fast/cuckoo_fast.cu:306-323, 595-622).  The row is in the own
     // slots; only the warp's slots below q are visited, which makes a query cost about n_j^2 / 2
     // products instead of n_j L.  Each warp leaves its sum at QS[j][warp] in shared memory;
-    // fold_queries combines them after the next barrier.
+    // fold_last combines them after the next barrier.
     // ---------------------------------------------------------------------------------------
     CF_HD void query_row(int q) {
-        u64* qs = sm + SM::QS;
         constexpr int U = E < 4 ? E : 4;  // slots a turn; the next turn's inverses load meanwhile
-        for (int jq = 0; jq < kp.J; ++jq) {
-            const int nj = kp.qn[jq], Mj = kp.qM[jq];
-            if (nj < q) continue;
+        this->each_query(q, [&](int jq, u64* qs) CF_INL {
+            const int Mj = kp.qM[jq];
             ex.each([&](int t, Regs<G>&) CF_INL {
                 const FpMod m = fm();
                 const double* iv = invd() + (Mj - t);  // 1/(M_j - w) of slot j's w = t + jT sits at iv - jT
@@ -740,9 +738,9 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
                     }
                     acc = fp_red(acc, m);  // at most four terms below 0.6p and the sum below 0.51p
                 }
-                ex.warp_sum_store(lt(t), fp_canon(acc, m), P, qs + (size_t)jq * NW, 1);
+                ex.warp_sum_store(lt(t), fp_canon(acc, m), P, qs, 1);
             });
-        }
+        });
     }
 
     // body(j, entry of own slot j, D[i - off], lo <= i < hi) over the slots j whose index i = t + jT lies in
@@ -872,7 +870,7 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
         if (n > d0) {  // the last row n, left in the own slots, for queries with n_j = n
             query_row(n);
             ex.sync();
-            fold_queries(n);
+            fold_last(n);
         }
         csync();  // every CTA's row sums are in
         if (rank() == 0) {  // in a cluster, the first CTA adds up the CTAs' row sums

@@ -42,7 +42,7 @@ struct PrimeRun<G, X, true> : PrimeBase<G, X, 1> {
     using Base::sum_red;
     using Base::warp_slot_range;
     using Base::load_row;
-    using Base::fold_queries;
+    using Base::fold_last;
     // L = 2^14 (1024 threads x 16 entries): the kernel spectrum lives in tensor memory, each
     // thread's 16 (value, companion) pairs in its own 64 columns (all 512 columns of the SM's 128
     // lanes); smaller transforms, several CTAs to an SM, read it from global.  A cluster's CTAs
@@ -584,14 +584,12 @@ struct PrimeRun<G, X, true> : PrimeBase<G, X, 1> {
     // registers (layout 0, entries outside the row zero).  Only the slots below q are visited: the
     // warp leaves the unrolled slot loop at its first slot wholly at or above q (slot indices grow
     // with j, so the exit is warp-uniform), which makes a query cost about n_j^2 / 2 products
-    // instead of n_j L.  Each warp leaves its sum at QS[j][warp] in shared memory; fold_queries
+    // instead of n_j L.  Each warp leaves its sum at QS[j][warp] in shared memory; fold_last
     // combines them after the next barrier.
     // ---------------------------------------------------------------------------------------
     CF_HD void query_row(int q) {
-        u64* qs = sm + SM::QS;
-        for (int jq = 0; jq < kp.J; ++jq) {
-            const int nj = kp.qn[jq], Mj = kp.qM[jq];
-            if (nj < q) continue;
+        this->each_query(q, [&](int jq, u64* qs) CF_INL {
+            const int Mj = kp.qM[jq];
             ex.each([&](int t, Regs<G>& rg) CF_INL {
                 const u64* iv = inv() + 2 * (size_t)Mj;  // the pair of 1/(M_j - w) sits at iv - 2w
                 const int tw = t & ~31;                  // the warp's first thread
@@ -631,9 +629,9 @@ struct PrimeRun<G, X, true> : PrimeBase<G, X, 1> {
                     }
                 }
                 const u64 part = canon(shoup_mul_lazy(acc, 1, misc()[MI_ONEQ], P));
-                ex.warp_sum_store(lt(t), part, P, qs + (size_t)jq * NW, 1);
+                ex.warp_sum_store(lt(t), part, P, qs, 1);
             });
-        }
+        });
     }
     // One step of the suffix recurrence (fast/cuckoo_fast.cu:841-855).
     CF_HD void step(int v) {
@@ -669,7 +667,7 @@ struct PrimeRun<G, X, true> : PrimeBase<G, X, 1> {
                     },
                     [&](auto jc) CF_INL { pin(rg.x[decltype(jc)::value]); });
             });
-            fold_queries(v);  // after the transform's barriers: every warp's partial of row v is in
+            fold_last(v);  // after the transform's barriers: every warp's partial of row v is in
         }
         if (v >= d0) {  // stage 2: column v of V from row v of S
             csync();  // column v of S is read below
@@ -764,7 +762,7 @@ struct PrimeRun<G, X, true> : PrimeBase<G, X, 1> {
             ex.each([&](int t, Regs<G>& rg) CF_INL { load_row(t, rg.x, V(), VS(), n, d0, n); });
             query_row(n);
             ex.sync();
-            fold_queries(n);
+            fold_last(n);
         }
         csync();  // every CTA's row sums are in
         if (rank() == 0) {  // in a cluster, the first CTA adds up the CTAs' row sums

@@ -328,6 +328,7 @@ struct KParams {
     const long long* qout = nullptr;  // [J] output index of each query (work-queue items), or null
     u64* keep = nullptr;  // resident tables [B][keep_words] (serving builds), or null
     size_t keep_words = 0;
+    int JC = 0;  // queries whose partial sums shared memory holds at a time (0: all J)
 };
 
 // Error codes recorded in *err by the kernel.
@@ -361,8 +362,8 @@ struct Smem {
     // A cluster's CTAs take more than half an SM's shared memory, so no two share an SM (a CTA
     // waiting for tensor memory held by another CTA of its own cluster would never get it).
     static constexpr size_t BYTES = G::C > 1 && WORDS * 8 < 120 * 1024 ? 120 * 1024 : (size_t)WORDS * 8;
-    // [J][NW] per-warp query partial sums of the current row, after the fixed part (the launch's
-    // dynamic shared memory is BYTES + 8 J NW)
+    // [JC][NW] per-warp query partial sums of the current row, after the fixed part (the launch's
+    // dynamic shared memory is BYTES + 8 JC NW)
     static constexpr int QS = WORDS;
     static constexpr size_t bytes_for(int J) { return BYTES + (size_t)8 * J * G::NW; }
 };
@@ -492,18 +493,39 @@ struct PrimeBase {
         }
     }
 
-    // Row q's per-warp partials (written by query_row before a barrier) into ps[j][q]: warp w folds
-    // queries w, w + NW, ... with shuffles.
-    CF_HD void fold_queries(int q) {
+    // Row q's per-warp partials of queries ja .. jb - 1 (written before a barrier) into ps[j][q]: warp w
+    // folds queries ja + w, ja + w + NW, ... with shuffles.
+    CF_HD void fold_queries(int q, int ja, int jb) {
         const u64* qs = sm + SM::QS;
         ex.each([&](int t, Regs<G>&) CF_INL {
             const int w = lt(t) >> 5, lane = t & 31;
-            for (int jq = w; jq < kp.J; jq += NW) {
+            for (int jq = ja + w; jq < jb; jq += NW) {
                 if (kp.qn[jq] < q) continue;
-                const u64 v = lane < NW ? qs[(size_t)jq * NW + lane] : 0;
+                const u64 v = lane < NW ? qs[(size_t)(jq - ja) * NW + lane] : 0;
                 ex.warp_sum_store(lt(t), v, P, ps() + (size_t)jq * (kp.n + 1) + q, 0);
             }
         });
+    }
+    // one(jq, where the warps' partials go) for every query with n_j >= q, JC at a time: all but the last
+    // batch are folded here, the last by fold_last after the caller's next barrier.
+    CF_HD int query_batch() const { return kp.JC > 0 && kp.JC < kp.J ? kp.JC : kp.J; }
+    template <class F>
+    CF_HD void each_query(int q, F&& one) {
+        const int jc = query_batch();
+        for (int ja = 0; ja < kp.J;) {
+            const int jb = ja + jc < kp.J ? ja + jc : kp.J;
+            for (int jq = ja; jq < jb; ++jq)
+                if (kp.qn[jq] >= q) one(jq, sm + SM::QS + (size_t)(jq - ja) * NW);
+            ja = jb;
+            if (jb < kp.J) {
+                ex.sync();
+                fold_queries(q, jb - jc, jb);
+                ex.sync();
+            }
+        }
+    }
+    CF_HD void fold_last(int q) {
+        if (kp.J > 0) fold_queries(q, (kp.J - 1) / query_batch() * query_batch(), kp.J);
     }
 
     // The full tile's columns v0 .. v0 + 15 into row storage, the thread's own rows r = t + jT (rows of later

@@ -37,15 +37,14 @@ struct cf_uneven {
 
 namespace {
 
-// Queries per table the launch's shared memory holds at transform length 2^lg.
+// Queries per table a launch takes at transform length 2^lg.
 int jcap_for(int lg, bool wide) {
     const KInfo ki = kernel_for(lg, wide);
     int dev = 0, optin = 0;
     if (!ki.fn || cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         return 0;
-    const int nw = ki.threads >= 32 ? ki.threads / 32 : 1;
-    return optin > (int)ki.smem ? (int)((optin - ki.smem) / (8 * (size_t)nw)) : 0;
+    return query_cap(lg, ki, optin);
 }
 
 void destroy(cf_uneven* u) {
@@ -131,6 +130,7 @@ int cf_uneven_create(cf_engine* e, const int* n, const int* M, const int* d, int
             long slots;
             KInfo ki;
             size_t smem;
+            int JC;  // queries summed at a time
         };
         std::vector<Group> gs;
         int sms = 0, dev = e->device;
@@ -139,7 +139,7 @@ int cf_uneven_create(cf_engine* e, const int* n, const int* M, const int* d, int
         long slots_max = 0;
         for (size_t a = 0; a < T;) {
             size_t b = a;
-            Group g{pl.tables[a].lg, a, a, 0, 0, 0, Layout(), 0, KInfo(), 0};
+            Group g{pl.tables[a].lg, a, a, 0, 0, 0, Layout(), 0, KInfo(), 0, 0};
             while (b < T && pl.tables[b].lg == g.lg) {
                 g.nmax = std::max(g.nmax, pl.tables[b].n);
                 g.F = std::max(g.F, pl.tables[b].F);
@@ -151,8 +151,7 @@ int cf_uneven_create(cf_engine* e, const int* n, const int* M, const int* d, int
             if (!g.ki.qfn) return fail(e, CF_ERR_UNSUPPORTED, "no kernel for this transform length");
             const int nw = g.ki.threads >= 32 ? g.ki.threads / 32 : 1;
             g.lay = make_layout(g.nmax, g.F, 1 << g.lg, g.J, nw, g.ki.r);
-            g.smem = g.ki.smem_for(g.J);
-            int rc = check_smem(e, g.smem, g.J);
+            int rc = plan_queries(e, g.lg, g.ki, g.J, &g.smem, &g.JC);
             if (rc) return rc;
             CF_CUDA(cudaFuncSetAttribute((const void*)g.ki.qfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem),
                     "shared memory attribute");
@@ -188,6 +187,7 @@ int cf_uneven_create(cf_engine* e, const int* n, const int* M, const int* d, int
             kp.lay = g.lay;
             kp.out = u->d_out;
             kp.err = u->d_err;
+            kp.JC = g.JC;
             QueueParams qp;
             qp.items = u->d_items + g.a;
             qp.count = (int)(g.b - g.a);

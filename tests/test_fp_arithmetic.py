@@ -1,6 +1,6 @@
 """The double-precision modular arithmetic (fparith.cuh) against whole numbers, at the edges of its
-stated ranges, and the kernels' phase code in the default geometries for primes below 2^50 against
-the oracle, with every butterfly's bound checked (CF_CHECK_BOUNDS).  All on the CPU."""
+stated ranges, and the kernels' phase code in the default geometries against the oracle, with every
+double-precision butterfly's bound checked (CF_CHECK_BOUNDS).  All on the CPU."""
 import ctypes
 import os
 import subprocess
@@ -8,6 +8,7 @@ import subprocess
 import numpy as np
 import pytest
 
+import cuckoo_b200 as cb
 import helpers as h
 
 PRIMES = [1125899865948161, h.oracle_primes(0, 1)[0], 4293918721, 97]  # the top of the list, a library prime, a tiny one
@@ -65,15 +66,32 @@ def test_reductions(fp, p):
         assert int(fp.fp_power_small(float(p // 3), k, float(p))) % p == pow(p // 3, k, p)
 
 
-@pytest.mark.parametrize("lg,R,nmax", [
-    (14, 5, 70), (11, 3, 1025), (10, 3, 1024), (10, 2, 600), (9, 3, 512), (9, 2, 257), (9, 2, 512),
-    (8, 2, 255), (8, 1, 256), (8, 1, 129), (7, 1, 128), (7, 1, 65),
+@pytest.mark.parametrize("lg,R,nmax,bits", [
+    (14, 5, 70, 50), (11, 3, 1025, 50), (10, 3, 1024, 50), (10, 2, 600, 50), (9, 3, 512, 50), (9, 2, 257, 50), (9, 2, 512, 50),
+    (8, 2, 255, 50), (8, 1, 256, 50), (8, 1, 129, 50), (7, 1, 128, 50), (7, 1, 65, 50),
+    (13, 3, 90, 62), (12, 3, 80, 62), (11, 2, 1025, 62), (10, 2, 600, 62), (9, 2, 512, 62), (8, 2, 129, 62), (7, 1, 128, 62),
 ])
-def test_default_geometries_match_oracle(fp, lg, R, nmax):
-    p = h.oracle_primes(0, 1)[0]
+def test_default_geometries_match_oracle(fp, lg, R, nmax, bits):
+    p = cb.prime_range(0, 1, bits=bits)[0]
     for model, d in ((0, 3), (1, 2)):
         qs = [(nmax, 2 * nmax + 1), (max(d, nmax // 3), nmax)]
-        qn, qM = (ctypes.c_int * 2)(*[q[0] for q in qs]), (ctypes.c_int * 2)(*[q[1] for q in qs])
-        out = (ctypes.c_uint64 * 2)()
-        rc = fp.emu_fp_geo(ctypes.c_uint64(p), nmax, d, model, qn, qM, 2, out, lg, R)
-        assert rc == 0 and [int(x) for x in out] == h.oracle_residues(p, nmax, d, qs, model)
+        assert run_geo(fp, p, nmax, d, model, qs, lg, R, 0) == h.oracle_residues(p, nmax, d, qs, model)
+
+
+def run_geo(fp, p, nmax, d, model, qs, lg, R, JC):
+    J = len(qs)
+    qn, qM = (ctypes.c_int * J)(*[q[0] for q in qs]), (ctypes.c_int * J)(*[q[1] for q in qs])
+    out = (ctypes.c_uint64 * J)()
+    rc = fp.emu_fp_geo(ctypes.c_uint64(p), nmax, d, model, qn, qM, J, out, lg, R, JC)
+    assert rc == 0, rc
+    return [int(x) for x in out]
+
+
+@pytest.mark.parametrize("lg,R,bits", [(7, 1, 50), (12, 4, 50), (7, 1, 62), (12, 3, 62)])
+@pytest.mark.parametrize("JC", [1, 2, 3, 7])
+def test_queries_in_batches(fp, lg, R, bits, JC):
+    """More queries than shared memory holds partial sums for: the batches' folds give the same residues."""
+    p = cb.prime_range(2, 1, bits=bits)[0]
+    n = 60
+    qs = [(n - 7 * k, 2 * n + k) for k in range(7)]
+    assert run_geo(fp, p, n, 3, 0, qs, lg, R, JC) == h.oracle_residues(p, n, 3, qs)

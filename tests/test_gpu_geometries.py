@@ -26,3 +26,17 @@ def test_few_and_many_primes_agree(n, per_sm, model):
     if n <= 1025:
         for row, p in ((a[0], primes[0]), (b[-1], primes[-1])):
             assert [int(x) for x in row] == h.oracle_residues(p, n, d, qs, model)
+
+
+@pytest.mark.parametrize("n,J,bits", [(2100, 1600, 50), (1100, 3400, 50), (4100, 700, 62)])
+def test_more_queries_than_one_batch(n, J, bits):
+    """Launches whose queries' partial sums do not fit shared memory at once sum them in batches."""
+    primes = cb.prime_range(0, 2, bits=bits)
+    qs = [(n - k % n // 2, 2 * n + k % 50) for k in range(J)]
+    with cb.Engine(0) as eng:
+        got = eng.residues(primes, n, 3, qs)
+        want = np.concatenate([eng.residues(primes, n, 3, qs[a:a + 250]) for a in range(0, J, 250)], axis=1)
+        with pytest.raises(cb.EngineError) as e:
+            eng.residues(primes, n, 3, qs * 8)
+        assert e.value.code == cb.CF_ERR_UNSUPPORTED
+    assert np.array_equal(got, want)
