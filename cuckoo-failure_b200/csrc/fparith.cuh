@@ -87,14 +87,13 @@ CF_HD double fp_pow(double x, u64 e, const FpMod& m) {
     }
     return r;
 }
-// x^k for 0 <= k <= 32, the same by all lanes without divergence: each turn's two products are
-// independent, so the chain is six products deep
-CF_HD double fp_pow_small(double x, int k, const FpMod& m) {
+// x^k, |x| <= 0.75 p: each turn's two products are independent, so the chain is one product per bit of k
+CF_HD double fp_pow_fast(double x, int k, const FpMod& m) {
     double r = 1.0;
 #pragma unroll 1
-    for (int b = 0; b < 6; ++b) {
+    for (; k; k >>= 1) {
         const double y = fp_mulmod(r, x, m);
-        r = (k >> b) & 1 ? y : r;
+        r = k & 1 ? y : r;
         x = fp_mulmod(x, x, m);
     }
     return r;

@@ -6,9 +6,8 @@ cfb::KInfo cf_kinfo_lg10();
 int cf_kvariants_lg10(cfb::KInfo* out, int cap) {
     const cfb::KInfo v[] = {
         cf_kinfo_lg10(),
-        cfb::kinfo_geo<10, 3, 4>(),
-        cfb::kinfo_geo<10, 2, 2>(),
-        cfb::kinfo_geo<10, 4, 8>()};
+        cfb::kinfo_geo<10, 4, 8>(),
+        cfb::kinfo_geo<10, 2, 4>()};
     const int k = (int)(sizeof(v) / sizeof(v[0]));
     for (int i = 0; i < k && i < cap; ++i) out[i] = v[i];
     return k;

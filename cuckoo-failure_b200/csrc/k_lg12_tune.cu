@@ -6,8 +6,7 @@ cfb::KInfo cf_kinfo_lg12();
 int cf_kvariants_lg12(cfb::KInfo* out, int cap) {
     const cfb::KInfo v[] = {
         cf_kinfo_lg12(),
-        cfb::kinfo_geo<12, 4, 2>(),
-        cfb::kinfo_geo<12, 3, 1>(),
+        cfb::kinfo_geo<12, 3, 2>(),
         cfb::kinfo_geo<12, 5, 4>()};
     const int k = (int)(sizeof(v) / sizeof(v[0]));
     for (int i = 0; i < k && i < cap; ++i) out[i] = v[i];

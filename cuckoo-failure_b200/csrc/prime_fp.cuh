@@ -410,34 +410,22 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
     // h = 1/g(v + 1) for the next step's row of S, both built behind the first barrier of step v's
     // second convolution.  A[k] = h^k (k < TA = min(CT, 32)), B[k] = h^(TA k) (k < TB = CT / TA),
     // J[j] = h^(T j) (j < E) and h^L.  Slot j of thread t holds index t + jT, whose power is
-    // A[t % TA] B[t / TA] J[j].  The groups (A, B, J for two bases) go to six warps, fewer warps
-    // looping over them; a group's lanes raise a common base (h, h^TA or h^T, which every lane squares
-    // up itself) to their own small exponent.  In a cluster, t is the thread's index in its CTA and
-    // J[j] = h^(c CT + T j) carries the CTA's offset c CT.
-    static constexpr int TA = CT < 32 ? CT : 32, TB = CT / TA;
-    static constexpr int LW = CT < 32 ? CT : 32;  // lanes of a warp
+    // A[t % TA] B[t / TA] J[j].  Every entry is a power by its own thread (the first 2 PWN threads, fewer
+    // taking several), a chain as long as its exponent's bits.  In a cluster, t is the thread's index in
+    // its CTA and J[j] = h^(c CT + T j) carries the CTA's offset c CT.
+    static constexpr int TA = CT < 32 ? CT : 32, TB = CT / TA, PWN = TA + TB + E + 1;
     CF_HD void power_tables(int t, int v) {
         double* pw = (double*)(sm + SM::PW);
         const FpMod m = fm();
-        const int lane = t & 31;
-        for (int gi = lt(t) >> 5; gi < 6; gi += NW) {
-            const int bs = gi & 1, kind = gi >> 1;
-            const int size = kind == 0 ? TA : kind == 1 ? TB : E + 1;
-            if (lane >= size) continue;
-            double* tab = pw + bs * SM::PW_STRIDE;
-            double h = ldd(Gd() + 2 * v + (bs ? 0 : 3));  // g(v) or 1/g(v + 1)
-            double off = 1.0;                       // h^(c CT): the CTA's offset (clusters)
-            if constexpr (C > 1)
-                if (kind == 2 && rank() > 0) off = fp_pow(h, (u64)rank() * CT, m);
-            const int sq = kind == 0 ? 0 : kind == 1 ? lg2(TA) : lg2(T);
-            for (int i = 0; i < sq; ++i) h = fp_mulmod(h, h, m);
-            for (int k = lane; k < size; k += LW) {
-                const double y = fp_pow_small(h, k, m);
-                if (kind == 0) tab[PW_A + k] = y;
-                else if (kind == 1) tab[PW_B + k] = y;
-                else if (k < E) tab[PW_J + k] = C > 1 ? fp_mulmod(y, off, m) : y;
-                else tab[PW_L] = y;
-            }
+        for (int x = lt(t); x < 2 * PWN; x += CT) {
+            const int bs = x >= PWN, y = x - bs * PWN;
+            int slot, e;
+            if (y < TA) slot = PW_A + y, e = y;
+            else if (y < TA + TB) slot = PW_B + (y - TA), e = TA * (y - TA);
+            else if (y < TA + TB + E) slot = PW_J + (y - TA - TB), e = T * (y - TA - TB) + rank() * CT;
+            else slot = PW_L, e = L;
+            const double h = ldd(Gd() + 2 * v + (bs ? 0 : 3));  // g(v) or 1/g(v + 1)
+            pw[bs * SM::PW_STRIDE + slot] = fp_pow_fast(h, e, m);
         }
     }
     // the thread's part A[t % TA] B[t / TA] of its slots' powers, and the table J of the slots'
@@ -710,36 +698,87 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
     // fold_last combines them after the next barrier.
     // ---------------------------------------------------------------------------------------
     CF_HD void query_row(int q) {
-        constexpr int U = E < 4 ? E : 4;  // slots a turn; the next turn's inverses load meanwhile
-        this->each_query(q, [&](int jq, u64* qs) CF_INL {
-            const int Mj = kp.qM[jq];
-            ex.each([&](int t, Regs<G>&) CF_INL {
-                const FpMod m = fm();
-                const double* iv = invd() + (Mj - t);  // 1/(M_j - w) of slot j's w = t + jT sits at iv - jT
-                const int tw = t & ~31;
-                auto get = [&](double (&c)[U], int j0) CF_INL {  // zero past the row
+        this->query_batches(q, [&](int ja, int jb, u64* qs) CF_INL {
+            int at[4], cnt = 0;
+            for (int jq = ja; jq < jb; ++jq) {
+                if (kp.qn[jq] >= q) at[cnt++] = jq;
+                if (cnt == 4 || (jq + 1 == jb && cnt > 2)) query_group<4>(q, at, cnt, qs - (ptrdiff_t)ja * NW), cnt = 0;
+            }
+            if (cnt == 2) query_group<2>(q, at, cnt, qs - (ptrdiff_t)ja * NW);
+            else if (cnt == 1) query_group<1>(q, at, cnt, qs - (ptrdiff_t)ja * NW);
+        });
+    }
+    // NJ queries at a time (at[0 .. cnt - 1]): an entry is read once for all of them, and their loads,
+    // products and warp sums overlap.  qs: where query 0's partials would go.
+    template <int NJ>
+    CF_HD void query_group(int q, const int (&at)[4], int cnt, u64* qs) {
+        constexpr int U = E < 4 ? E : NJ > 2 ? 2 : 4;  // slots a turn; the next turn's inverses load meanwhile
+        int M[NJ];
 #pragma unroll
-                    for (int k = 0; k < U; ++k) {
-                        c[k] = 0;
-                        if (t + (j0 + k) * T < q) c[k] = ldt(iv - (j0 + k) * T);
+        for (int k = 0; k < NJ; ++k) M[k] = k < cnt ? kp.qM[at[k]] : -1;
+        ex.each([&](int t, Regs<G>&) CF_INL {
+            const FpMod m = fm();
+            const double* iv = invd() - t;  // 1/(M - w) of slot j's w = t + jT sits at iv + M - jT
+            const int tw = t & ~31;
+            auto get = [&](double (&c)[NJ][U], int j0) CF_INL {  // zero past the row and for queries left out
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int k = 0; k < NJ; ++k) {
+                        c[k][u] = 0;
+                        if (t + (j0 + u) * T < q && M[k] >= 0) c[k][u] = ldt(iv + M[k] - (j0 + u) * T);
                     }
-                };
-                double acc = 0, c[U];
-                get(c, 0);
+            };
+            double acc[NJ], c[NJ][U];
+#pragma unroll
+            for (int k = 0; k < NJ; ++k) acc[k] = 0;
+            get(c, 0);
 #pragma unroll 1
-                for (int j0 = 0; j0 < E && tw + j0 * T < q; j0 += U) {
-                    double next[U];
-                    get(next, j0 + U);
+            for (int j0 = 0; j0 < E && tw + j0 * T < q; j0 += U) {
+                double next[NJ][U];
+                get(next, j0 + U);
 #pragma unroll
-                    for (int k = 0; k < U; ++k) {
-                        const double x = tw + (j0 + k) * T < q ? fp_bits(sm[own(t, j0 + k)]) : 0.0;
-                        acc = fp_add(acc, fp_mulmod(x, c[k], m));
-                        c[k] = next[k];
-                    }
-                    acc = fp_red(acc, m);  // at most four terms below 0.6p and the sum below 0.51p
+                for (int u = 0; u < U; ++u) {
+                    const double x = tw + (j0 + u) * T < q ? fp_bits(sm[own(t, j0 + u)]) : 0.0;
+#pragma unroll
+                    for (int k = 0; k < NJ; ++k) acc[k] = fp_add(acc[k], fp_mulmod(x, c[k][u], m)), c[k][u] = next[k][u];
                 }
-                ex.warp_sum_store(lt(t), fp_canon(acc, m), P, qs, 1);
-            });
+#pragma unroll
+                for (int k = 0; k < NJ; ++k) acc[k] = fp_red(acc[k], m);  // at most four terms below 0.6p and the sum below 0.51p
+            }
+#if defined(__CUDA_ARCH__)
+            // the warp's sums: while a lane holds several, each exchange halves them (lane bit 4, then 3, picks
+            // the query); at most three additions of values below 0.51p between reductions
+            const unsigned mask = CT >= 32 ? 0xffffffffu : (1u << CT) - 1u;
+            constexpr int O0 = CT >= 32 ? 16 : CT / 2;
+            if constexpr (NJ == 4 && CT >= 32) {
+                const int lane = t & 31;
+                const bool up = lane & 16, up2 = lane & 8;
+                const double a0 = fp_add(up ? acc[2] : acc[0], __shfl_xor_sync(mask, up ? acc[0] : acc[2], 16));
+                const double a1 = fp_add(up ? acc[3] : acc[1], __shfl_xor_sync(mask, up ? acc[1] : acc[3], 16));
+                double a = fp_add(up2 ? a1 : a0, __shfl_xor_sync(mask, up2 ? a0 : a1, 8));
+                a = fp_add(a, __shfl_xor_sync(mask, a, 4));
+                a = fp_red(a, m);
+                a = fp_add(a, __shfl_xor_sync(mask, a, 2));
+                a = fp_add(a, __shfl_xor_sync(mask, a, 1));
+                const int k = lane >> 3;  // 2 (bit 4) + (bit 3)
+                const int j = k == 0 ? at[0] : k == 1 ? at[1] : k == 2 ? at[2] : at[3];
+                if ((lane & 7) == 0 && k < cnt) qs[(ptrdiff_t)j * NW + (lt(t) >> 5)] = fp_canon(a, m);
+            } else {
+#pragma unroll
+                for (int k = 0; k < NJ; ++k) {
+                    double a = acc[k];
+#pragma unroll
+                    for (int o = O0; o >= 1; o >>= 1) {
+                        a = fp_add(a, __shfl_xor_sync(mask, a, o));
+                        if (o == 4) a = fp_red(a, m);
+                    }
+                    if ((t & 31) == 0 && k < cnt) qs[(ptrdiff_t)at[k] * NW + (lt(t) >> 5)] = fp_canon(a, m);
+                }
+            }
+#else
+            for (int k = 0; k < NJ && k < cnt; ++k) ex.warp_sum_store(lt(t), fp_canon(acc[k], m), P, qs + (ptrdiff_t)at[k] * NW, 1);
+#endif
         });
     }
 

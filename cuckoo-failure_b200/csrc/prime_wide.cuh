@@ -588,8 +588,11 @@ struct PrimeRun<G, X, true> : PrimeBase<G, X, 1> {
     // combines them after the next barrier.
     // ---------------------------------------------------------------------------------------
     CF_HD void query_row(int q) {
-        this->each_query(q, [&](int jq, u64* qs) CF_INL {
-            const int Mj = kp.qM[jq];
+        this->query_batches(q, [&](int ja, int jb, u64* qs0) CF_INL {
+          for (int jq = ja; jq < jb; ++jq) {
+            const int nj = kp.qn[jq], Mj = kp.qM[jq];
+            u64* qs = qs0 + (size_t)(jq - ja) * NW;
+            if (nj < q) continue;
             ex.each([&](int t, Regs<G>& rg) CF_INL {
                 const u64* iv = inv() + 2 * (size_t)Mj;  // the pair of 1/(M_j - w) sits at iv - 2w
                 const int tw = t & ~31;                  // the warp's first thread
@@ -631,6 +634,7 @@ struct PrimeRun<G, X, true> : PrimeBase<G, X, 1> {
                 const u64 part = canon(shoup_mul_lazy(acc, 1, misc()[MI_ONEQ], P));
                 ex.warp_sum_store(lt(t), part, P, qs, 1);
             });
+          }
         });
     }
     // One step of the suffix recurrence (fast/cuckoo_fast.cu:841-855).

@@ -493,33 +493,31 @@ struct PrimeBase {
         }
     }
 
-    // Row q's per-warp partials of queries ja .. jb - 1 (written before a barrier) into ps[j][q]: warp w
-    // folds queries ja + w, ja + w + NW, ... with shuffles.
+    // Row q's per-warp partials of queries ja .. jb - 1 (written before a barrier) into ps[j][q], a thread
+    // per query.  A query with n_j < q has none: its word of row q is never read.
     CF_HD void fold_queries(int q, int ja, int jb) {
         const u64* qs = sm + SM::QS;
         ex.each([&](int t, Regs<G>&) CF_INL {
-            const int w = lt(t) >> 5, lane = t & 31;
-            for (int jq = ja + w; jq < jb; jq += NW) {
-                if (kp.qn[jq] < q) continue;
-                const u64 v = lane < NW ? qs[(size_t)(jq - ja) * NW + lane] : 0;
-                ex.warp_sum_store(lt(t), v, P, ps() + (size_t)jq * (kp.n + 1) + q, 0);
+            for (int jq = ja + lt(t); jq < jb; jq += CT) {
+                u64 s = 0;
+#pragma unroll 4
+                for (int w = 0; w < NW; ++w) s = madd(s, qs[(size_t)(jq - ja) * NW + w], P);
+                ps()[(size_t)jq * (kp.n + 1) + q] = s;
             }
         });
     }
-    // one(jq, where the warps' partials go) for every query with n_j >= q, JC at a time: all but the last
-    // batch are folded here, the last by fold_last after the caller's next barrier.
+    // some(ja, jb, where the warps' partials of query ja go) for ranges of the queries, JC at a time: all
+    // but the last batch are folded here, the last by fold_last after the caller's next barrier.
     CF_HD int query_batch() const { return kp.JC > 0 && kp.JC < kp.J ? kp.JC : kp.J; }
     template <class F>
-    CF_HD void each_query(int q, F&& one) {
+    CF_HD void query_batches(int q, F&& some) {
         const int jc = query_batch();
-        for (int ja = 0; ja < kp.J;) {
+        for (int ja = 0; ja < kp.J; ja += jc) {
             const int jb = ja + jc < kp.J ? ja + jc : kp.J;
-            for (int jq = ja; jq < jb; ++jq)
-                if (kp.qn[jq] >= q) one(jq, sm + SM::QS + (size_t)(jq - ja) * NW);
-            ja = jb;
+            some(ja, jb, sm + SM::QS);
             if (jb < kp.J) {
                 ex.sync();
-                fold_queries(q, jb - jc, jb);
+                fold_queries(q, ja, jb);
                 ex.sync();
             }
         }

@@ -22,7 +22,7 @@ void fp_reductions(const double* x, double p, long n, double* out, uint64_t* can
     const FpMod m{p, 1.0 / p};
     for (long i = 0; i < n; ++i) out[i] = fp_red(x[i], m), canon[i] = fp_canon(x[i], m);
 }
-double fp_power_small(double x, int k, double p) { return fp_pow_small(x, k, FpMod{p, 1.0 / p}); }
+double fp_power_fast(double x, int k, double p) { return fp_pow_fast(x, k, FpMod{p, 1.0 / p}); }
 
 // one prime's residues with 2^R entries per thread and the transform length forced to 2^lg, the
 // queries' partial sums held JC at a time (0: all)

@@ -23,8 +23,8 @@ def fp(tmp_path_factory):
     L = ctypes.CDLL(so)
     L.fp_products.argtypes = [_dp, _dp, ctypes.c_double, ctypes.c_long, _dp]
     L.fp_reductions.argtypes = [_dp, ctypes.c_double, ctypes.c_long, _dp, _up]
-    L.fp_power_small.argtypes = [ctypes.c_double, ctypes.c_int, ctypes.c_double]
-    L.fp_power_small.restype = ctypes.c_double
+    L.fp_power_fast.argtypes = [ctypes.c_double, ctypes.c_int, ctypes.c_double]
+    L.fp_power_fast.restype = ctypes.c_double
     return L
 
 
@@ -62,8 +62,8 @@ def test_reductions(fp, p):
     fp.fp_reductions(xs.ctypes.data_as(_dp), float(p), len(xs), out.ctypes.data_as(_dp), canon.ctypes.data_as(_up))
     for u, r, c in zip(xs, out, canon):
         assert (int(r) - int(u)) % p == 0 and abs(r) <= 0.51 * p and int(c) == int(u) % p, (u, r, c)
-    for k in range(33):
-        assert int(fp.fp_power_small(float(p // 3), k, float(p))) % p == pow(p // 3, k, p)
+    for k in list(range(33)) + [1000, 16384]:
+        assert int(fp.fp_power_fast(float(p // 3), k, float(p))) % p == pow(p // 3, k, p)
 
 
 @pytest.mark.parametrize("lg,R,nmax,bits", [
