@@ -33,7 +33,9 @@ sys.path.insert(0, PKG)
 
 METRIC = "prime-residues/s, n=16384 d=3 NTT suffix build; served-query p50/p99 latency"
 UNIT = "prime-residues/s"
-K_OPS_PER_MM = 20  # INT32 multiply ops per 64-bit modular multiplication (fixed accounting model)
+# Operations per modular multiplication by prime bits (fixed accounting model): below 2^50 a product is six
+# double-precision operations and a butterfly adds two; below 2^62 a Shoup product is 20 INT32 multiplies.
+OPS_PER_MM = {50: (8, "fp64", "Top/s (FP64 instructions' lanes)"), 62: (20, "int32", "Top/s (INT32 IMAD)")}
 # DRAM bytes (read + write) per prime of the engine kernel, from an ncu capture of this bench at 2
 # primes per launch (profiles/k_suffix_n16384_b2_sections.md), keyed by (n, M, d, prime bits); the
 # bench scales it by the primes per launch
@@ -353,7 +355,7 @@ def config2_run(device, n=4096, M=8192, d=3, waves=4, reps=3):
             for i, r in gold.items():
                 assert int(got[i]) == r, f"config 2 ({label}): residue mismatch at prime {i}"
             out[label] = {"geometry": rec["variants"][k], "value": B / (ms * 1e-3), "unit": UNIT, "ms_per_launch": ms,
-                          "frac_top": B * algorithmic_mm(n) * K_OPS_PER_MM / (ms * 1e-3) / 1e12}
+                          "frac_top": B * algorithmic_mm(n) * OPS_PER_MM[50][0] / (ms * 1e-3) / 1e12}
     return out
 
 
@@ -385,7 +387,7 @@ def sweep_run(eng, n, M, B, reps=2):
         key = f"d{d}" + ("_replacement" if model else "") + ("_62bit" if bits == 62 else "")
         out[key] = {"value": B / (ms * 1e-3), "unit": UNIT, "ms_per_step": ms, "steps": reps,
                     "primes_needed": cb.need(n, M, d, model, bits=bits),
-                    "frac": B * algorithmic_mm(n) * K_OPS_PER_MM / (ms * 1e-3) / 1e12}
+                    "bits": bits, "frac": B * algorithmic_mm(n) * OPS_PER_MM[bits][0] / (ms * 1e-3) / 1e12}
     assert cb.lib().cf_engine_set_prime_bits(eng._h, 50) == 0
     return out
 
@@ -611,11 +613,14 @@ def main():
                  "what": "one launch per prime (batch of 1), same n, M, d and kernel, timed alone"}
 
     probe = ctypes.CDLL(os.path.join(PKG, "lib", "libcuckoo_b200_probe.so"))
-    probe.cfp_imad_ops_per_s.restype = ctypes.c_double
-    probe.cfp_imad_ops_per_s.argtypes = [ctypes.c_int, ctypes.c_int]
-    peak = probe.cfp_imad_ops_per_s(local, 5) / 1e12
+    peaks = {}
+    for bits, f in ((50, probe.cfp_dfma_ops_per_s), (62, probe.cfp_imad_ops_per_s)):
+        f.restype, f.argtypes = ctypes.c_double, [ctypes.c_int, ctypes.c_int]
+        peaks[bits] = f(local, 5) / 1e12
+    peak = peaks[a.prime_bits]
+    ops_mm, bound, ops_unit = OPS_PER_MM[a.prime_bits]
     # the timed stream holds only this engine's launches, back to back: per-GPU algorithmic rate
-    achieved = B * a.steps * algorithmic_mm(n) * K_OPS_PER_MM / (ms * 1e-3) / 1e12
+    achieved = B * a.steps * algorithmic_mm(n) * ops_mm / (ms * 1e-3) / 1e12
     per_prime = MEASURED_TRAFFIC_PER_PRIME.get((n, M, d, a.prime_bits))
     traffic = a.traffic_bytes or (per_prime * B if per_prime else None)
     hbm = None
@@ -643,13 +648,14 @@ def main():
         with cb.Engine(local) as eng2:
             out = sweep_run(eng2, n, M, B)
         for v in out.values():
-            v["frac"] = v["frac"] / peak if peak else None
+            bits = v.pop("bits")
+            v["frac"] = v["frac"] / peaks[bits] if peaks[bits] else None
         return out
 
     def cfg2_fn():
         out = config2_run(local)
         for k in ("default", "tuned"):
-            out[k]["frac"] = out[k].pop("frac_top") / peak if peak else None
+            out[k]["frac"] = out[k].pop("frac_top") / peaks[50] if peaks[50] else None
         return out
 
     def uneven_fn():
@@ -673,10 +679,10 @@ def main():
             "dtype": "u64", "data": "synthetic",
             "config": {"workload": workload, "batch_primes_per_step": B, "queries_per_prime": J,
                        "l2": "inputs larger than L2 (per-prime tables total far above 126 MB)"},
-            "roofline": {"bound": "int32", "achieved": achieved, "peak": peak, "unit": "Top/s (INT32 IMAD)",
+            "roofline": {"bound": bound, "achieved": achieved, "peak": peak, "unit": ops_unit,
                          "frac": achieved / peak if peak else None,
                          "traffic": traffic, "hbm": hbm,
-                         "model": f"{K_OPS_PER_MM} INT32 multiply ops per modular multiplication, "
+                         "model": f"{ops_mm} {bound} operations per modular multiplication, "
                                   f"{algorithmic_mm(n):.3e} multiplications per prime-residue; peak measured live"},
             "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches, "clocks": clk.summary(),
             "plain_form": plain, "config2": cfg2, "config3_sweep": sweep, "large_tables": large, "uneven": unev,

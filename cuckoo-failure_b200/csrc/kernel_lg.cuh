@@ -121,7 +121,7 @@ struct DevExec {
 //   2^14: 32 entries x 512 threads 703, 16 x 1024 853 (64 registers spill; n = 12500, 148 primes)
 //   2^13: 16 x 512, 128 registers 264; 32 x 256 371, 8 x 1024 297 (148 primes)
 //   2^12: 16 x 256 at 2 CTAs 238, 8 x 512 at 2 263, 32 x 128 at 4 329 (592 primes)
-//   2^11: 8 x 256 at 2 CTAs 132.5, at 4 (64 registers) 131, 16 x 128 at 4 139 (1184 primes)
+//   2^11: 8 x 256 at 3 CTAs 125, at 2 134, at 4 (64 registers, spills) 131, 16 x 128 at 4 139 (1184 primes)
 //   2^10: 8 x 128 at 4 CTAs 17.7, 4 x 256 at 2 21.1, at 4 19.6 (n = 1000, 592 primes)
 //   2^9:  8 x 64 at 8 CTAs 18.5, uncapped 23.2, 16 x 32 22.9 (2368 primes)
 //   2^8:  4 x 64 at 8 CTAs 5.6, uncapped 8.0, 8 x 32 6.7, 2 x 128 13.1 (2368 primes)
@@ -129,9 +129,9 @@ struct DevExec {
 // FEW: for batches of few primes, which leave SMs with one or two CTAs, more threads per prime shorten
 // a step; used up to few_per_sm(LG) primes per SM:
 //   2^12: 8 x 512 at 148 primes 69.9 against 78.2, at 200 138.6 against 120.5 (n = 4096): 1 per SM
-//   2^10: 4 x 256 at 296 primes 10.6 against 12.0, at 444 18.1 against 14.5 (n = 1000): 2 per SM
-//   2^9:  4 x 128 at 148 primes 3.5 against 4.8, at 592 7.7 against 6.3: 2 per SM
-//   2^8:  2 x 128 at 148 primes 1.56 against 1.76, at 592 3.4 against 2.2: 1 per SM
+//   2^10: 4 x 256 at 296 primes 10.7 against 12.0, at 360 17.9 against 14.5 (n = 1000): 2 per SM
+//   2^9:  4 x 128 at 296 primes 3.7 against 4.9, at 360 6.8 against 5.8 (n = 500): 2 per SM
+//   2^8:  2 x 128 at 296 primes 1.33 against 1.42, at 360 2.26 against 1.47 (n = 200): 2 per SM
 //
 // Primes below 2^62 (64-bit integers), one CTA's registers uncapped (ms per launch, n = 2^LG or the
 // stated n; in front the geometries with half to an eighth of the threads that were the default):
@@ -153,14 +153,14 @@ struct Geometry {
     static constexpr int MB = W          ? 1
                               : LG >= 13 ? 1
                               : LG == 12 ? (FEW ? 1 : 2)
-                              : LG == 11 ? 2
+                              : LG == 11 ? 3
                               : LG == 10 ? (FEW ? 2 : 4)
                               : LG == 9  ? (FEW ? 1 : 8)
                               : LG == 8  ? (FEW ? 1 : 8)
                               : LG == 7  ? 8
                                          : 1;
 };
-constexpr int few_per_sm(int lg) { return lg == 12 || lg == 8 ? 1 : lg == 10 || lg == 9 ? 2 : 0; }
+constexpr int few_per_sm(int lg) { return lg == 12 ? 1 : lg >= 8 && lg <= 10 ? 2 : 0; }
 // MB: resident CTAs per SM the variant is compiled for (its register cap).
 template <int LG, int R, bool W, int MB>
 __global__ void __launch_bounds__(Geo<LG, R>::T, MB) k_suffix(KParams kp) {

@@ -870,7 +870,6 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
                 if (mine) check(x, BD::inv(LG)), st_stream(col + j * T, y);
                 if (t + j * T == v + 1) next(y);
             });
-            if (v - tile_v0(v) == TILE - 1 && v < n - 1) this->flush_rows(t, tile_v0(v));
             in.put(sm, t, [&](int, double x) CF_INL { return x; });
         });
     }
@@ -890,6 +889,14 @@ struct PrimeRun<G, X, false> : PrimeBase<G, X, 0> {
             convolve(stage == 1 ? v : v > d0 ? v + 1 : 0, v + stage - 1, n + stage - 1, n == L);
             if (stage == 1) stage1_out(v);
             else stage2_out(v);
+        }
+        if (v - tile_v0(v) == TILE - 1 && v < n - 1) {
+#if defined(__CUDA_ARCH__)
+            __syncwarp();  // the warp's columns of the tile are in
+#else
+            ex.sync();
+#endif
+            ex.each([&](int t, Regs<G>&) CF_INL { this->flush_rows(t, tile_v0(v)); });
         }
         csync();
         ex.each([&](int t, Regs<G>&) CF_INL {

@@ -526,34 +526,39 @@ struct PrimeBase {
         if (kp.J > 0) fold_queries(q, (kp.J - 1) / query_batch() * query_batch(), kp.J);
     }
 
-    // The full tile's columns v0 .. v0 + 15 into row storage, the thread's own rows r = t + jT (rows of later
-    // groups only: a row of this tile's group reads these columns from the tile).  The thread wrote
-    // the staged columns of these rows itself, so no barrier is needed before it, and the cells
-    // written were last read by an earlier step.  Whole 32-byte sectors (4 columns of a block row) are
-    // stored, and a row's 2 FL loads go out before its first store (the stores wait for them in order).
+    // The full tile's columns v0 .. v0 + 15 into row storage, the rows r = t + jT of the warp's threads (rows of
+    // later groups only: a row of this tile's group reads these columns from the tile).  The warp wrote
+    // the staged columns of these rows itself, so only its own threads need to meet before it, and the
+    // cells written were last read by an earlier step.  Four lanes take a row, four columns each, so a
+    // store instruction fills eight whole 128-byte lines (one row per lane wrote a sector of 32 lines:
+    // the flush was bound by those).
     CF_HD void flush_rows(int t, int v0) const {
-        constexpr int FL = CT >= 1024 ? 4 : 8;
-        const int n = kp.n, d0 = kp.d0, h = block_h(n);
+        constexpr int LPR = CT < 32 ? 1 : 4, RW = CT < 32 ? 1 : 8;  // lanes per row, rows of a warp at a time
+        const int n = kp.n, d0 = kp.d0, h = block_h(n), lane = t & 31;
         const size_t cs = (size_t)n + 1;  // tile column stride
         const int cS = d0 + 1 > v0 ? d0 + 1 - v0 : 0, cV = d0 > v0 ? d0 - v0 : 0;
-        for (int r = t + (v0 + TILE - t + T - 1) / T * T; r <= n; r += T) {
-            const size_t off = blk_off(r, v0, h);  // columns v0 + c at off + c
-            if (cS == 0) {
-                const u64 *sS = SS() + (r < n ? r : n - 1), *sV = VS() + r;
-                u64 a[FL], b[FL];
+        const int r0 = CT < 32 ? t : (t & ~31) + lane / LPR, c0 = CT < 32 ? 0 : (lane % LPR) * (TILE / LPR);
+        for (int rb = (v0 + TILE - (CT < 32 ? t : (t & ~31) + 31) + T - 1) / T * T; r0 + rb <= n; rb += T) {
 #pragma unroll
-                for (int c0 = 0; c0 < TILE; c0 += FL) {
+            for (int g = 0; g < (CT < 32 ? 1 : 32 / RW); ++g) {
+                const int r = r0 + rb + g * RW;
+                if (r < v0 + TILE || r > n) continue;
+                const size_t off = blk_off(r, v0, h);  // columns v0 + c at off + c
+                if (cS == 0) {
+                    const u64 *sS = SS() + (r < n ? r : n - 1) + c0 * cs, *sV = VS() + r + c0 * cs;
+                    u64 a[TILE / LPR], b[TILE / LPR];
 #pragma unroll
-                    for (int c = 0; c < FL; ++c) a[c] = lds<CG>(sS + (c0 + c) * cs), b[c] = lds<CG>(sV + (c0 + c) * cs);
+                    for (int c = 0; c < TILE / LPR; ++c) a[c] = lds<CG>(sS + c * cs), b[c] = lds<CG>(sV + c * cs);
 #pragma unroll
-                    for (int c = 0; c < FL; c += 4) {
+                    for (int c = 0; c < TILE / LPR; c += 4) {
                         if (r < n) st_stream4(S() + off + c0 + c, a[c], a[c + 1], a[c + 2], a[c + 3]);
                         st_stream4(V() + off + c0 + c, b[c], b[c + 1], b[c + 2], b[c + 3]);
                     }
+                } else {  // rows r < n of S: entries q = v0 .. v, written for q > d0; of V: w = v0 .. v, written for w >= d0
+                    const int ce = c0 + TILE / LPR;
+                    for (int c = c0 > cS ? c0 : cS; c < ce && r < n; ++c) st_stream(S() + off + c, lds<CG>(SS() + r + c * cs));
+                    for (int c = c0 > cV ? c0 : cV; c < ce; ++c) st_stream(V() + off + c, lds<CG>(VS() + r + c * cs));
                 }
-            } else {  // rows r < n of S: entries q = v0 .. v, written for q > d0; of V: w = v0 .. v, written for w >= d0
-                for (int c = cS; c < TILE && r < n; ++c) st_stream(S() + off + c, lds<CG>(SS() + r + c * cs));
-                for (int c = cV; c < TILE; ++c) st_stream(V() + off + c, lds<CG>(VS() + r + c * cs));
             }
         }
     }

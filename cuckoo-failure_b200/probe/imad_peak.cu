@@ -1,6 +1,6 @@
-// Roofline denominator probe: the device's sustained 32-bit integer multiply-add (IMAD) rate,
-// measured with independent mad.lo.u32 chains.  Separate library (libcuckoo_b200_probe.so) used
-// only by bench.py; the engine never calls it.
+// Roofline denominator probe: the device's sustained rates of 32-bit integer multiply-adds (IMAD) and of
+// double-precision FMAs, measured with independent chains.  Separate library
+// (libcuckoo_b200_probe.so) used only by bench.py; the engine never calls it.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -15,9 +15,21 @@ static __global__ void k_imad(uint32_t* out, int iters, uint32_t m) {
     for (int i = 0; i < 8; ++i) s ^= x[i];
     out[blockIdx.x * blockDim.x + threadIdx.x] = s;
 }
+static __global__ void k_dfma(uint32_t* out, int iters, uint32_t m) {
+    double x[8];
+    const double a = 1.0 + 1e-9 * m, b = 1e-3;
+    for (int i = 0; i < 8; ++i) x[i] = threadIdx.x * 7 + i;
+    for (int it = 0; it < iters; ++it) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) asm volatile("fma.rn.f64 %0, %0, %1, %2;" : "+d"(x[i]) : "d"(a), "d"(b));
+    }
+    double s = 0;
+    for (int i = 0; i < 8; ++i) s += x[i];
+    out[blockIdx.x * blockDim.x + threadIdx.x] = (uint32_t)(s != 0.0);
+}
 
-// Returns IMAD operations per second (0 on error), best of `reps` timed launches on `device`.
-extern "C" double cfp_imad_ops_per_s(int device, int reps) {
+// Operations per second of `kernel` (0 on error), best of `reps` timed launches on `device`.
+static double ops_per_s(void (*kernel)(uint32_t*, int, uint32_t), int device, int reps) {
     if (cudaSetDevice(device) != cudaSuccess) return 0;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -27,11 +39,11 @@ extern "C" double cfp_imad_ops_per_s(int device, int reps) {
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
-    k_imad<<<blocks, threads>>>(d, iters, 12345u);
+    kernel<<<blocks, threads>>>(d, iters, 12345u);
     double best = 0;
     for (int r = 0; r < reps; ++r) {
         cudaEventRecord(a);
-        k_imad<<<blocks, threads>>>(d, iters, 12345u);
+        kernel<<<blocks, threads>>>(d, iters, 12345u);
         cudaEventRecord(b);
         cudaEventSynchronize(b);
         float ms = 0;
@@ -44,3 +56,5 @@ extern "C" double cfp_imad_ops_per_s(int device, int reps) {
     cudaFree(d);
     return cudaGetLastError() == cudaSuccess ? best : 0;
 }
+extern "C" double cfp_imad_ops_per_s(int device, int reps) { return ops_per_s(k_imad, device, reps); }
+extern "C" double cfp_dfma_ops_per_s(int device, int reps) { return ops_per_s(k_dfma, device, reps); }

@@ -11,7 +11,7 @@ import helpers as h
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,per_sm", [(65, 0), (128, 0), (129, 1), (256, 1), (257, 2), (512, 2), (513, 2), (1024, 2), (1025, 0), (2049, 1)])
+@pytest.mark.parametrize("n,per_sm", [(65, 0), (128, 0), (129, 2), (256, 2), (257, 2), (512, 2), (513, 2), (1024, 2), (1025, 0), (2049, 1)])
 @pytest.mark.parametrize("model", [0, 1])
 def test_few_and_many_primes_agree(n, per_sm, model):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
