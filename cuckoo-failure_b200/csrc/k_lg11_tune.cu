@@ -7,7 +7,8 @@ int cf_kvariants_lg11(cfb::KInfo* out, int cap) {
     const cfb::KInfo v[] = {
         cf_kinfo_lg11(),
         cfb::kinfo_geo<11, 4, 4>(),
-        cfb::kinfo_geo<11, 2, 1>()};
+        cfb::kinfo_geo<11, 2, 1>(),
+        cfb::kinfo_geo<11, 4, 2>()};
     const int k = (int)(sizeof(v) / sizeof(v[0]));
     for (int i = 0; i < k && i < cap; ++i) out[i] = v[i];
     return k;

@@ -7,7 +7,8 @@ int cf_kvariants_lg12(cfb::KInfo* out, int cap) {
     const cfb::KInfo v[] = {
         cf_kinfo_lg12(),
         cfb::kinfo_geo<12, 3, 2>(),
-        cfb::kinfo_geo<12, 5, 4>()};
+        cfb::kinfo_geo<12, 5, 4>(),
+        cfb::kinfo_geo<12, 5, 2>()};
     const int k = (int)(sizeof(v) / sizeof(v[0]));
     for (int i = 0; i < k && i < cap; ++i) out[i] = v[i];
     return k;

@@ -22,7 +22,8 @@ DEFAULT_CACHE = os.environ.get("CF_TUNE_CACHE", os.path.join(os.path.expanduser(
 
 
 def _key(device_name, lg, B):
-    return f"{device_name}|lg={lg}|batch={B}"
+    # "fp64": a pick that was timed on the integer kernels is measured again
+    return f"{device_name}|fp64|lg={lg}|batch={B}"
 
 
 def tuned(engine, nmax, Mmax, d, B, cache=DEFAULT_CACHE, device_name=None):
