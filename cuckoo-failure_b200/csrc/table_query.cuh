@@ -39,11 +39,13 @@ struct TQParams {
 
 constexpr int TQ_THREADS = 256, TQ_WARPS = TQ_THREADS / 32, TQ_PER_SM = 2;
 constexpr int TQ_ROWS = 16, TQ_K = 8, TQ_COLS = 32 * TQ_K;  // a warp's tile: rows, columns per lane, columns
-constexpr int TQ_CLUSTER = 8;                               // CTAs per prime at most
+constexpr int TQ_CLUSTER = 4;                               // CTAs per prime at most
 // Shared memory: per query Q and the warps' sums, and (read from the first CTA) the CTAs' sums.
 inline size_t tq_smem_bytes(int J) { return 8 * (size_t)J * (1 + TQ_WARPS + TQ_CLUSTER); }
 // CTAs per prime: the number up to TQ_CLUSTER whose waves of resident CTAs leave the least idle (the
 // CTAs' shares are equal, so a launch lasts waves / S), with a block of rows for every warp.
+// Four at most: beside a plain rebuild that fills 96 SMs, clusters of eight find fewer places in what
+// each GPC has left (served requests with n in 513 .. 2048: p50 10.6 ms, p99 44; with four 5.9 and 28).
 inline int tq_ctas(int B, int nmax, int sms) {
     const long cap = (long)TQ_PER_SM * (sms > 0 ? sms : 1);
     int S = 1;
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(TQ_THREADS, TQ_PER_SM) k_table_query(TQParams 
     extern __shared__ __align__(16) double tq_sm[];
     const int S = tp.S, b = blockIdx.x / S, s = blockIdx.x % S, J = tp.J;
     const int t = threadIdx.x, warp = t >> 5;
+    if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // waited for before the first remote store
     double* Qs = tq_sm;                    // [J] candidate sets per item
     double* sums = tq_sm + J;              // [TQ_WARPS][J]
     double* all = sums + TQ_WARPS * J;     // [S][J], in the cluster's first CTA
@@ -165,6 +168,7 @@ __global__ void __launch_bounds__(TQ_THREADS, TQ_PER_SM) k_table_query(TQParams 
         at += tiles;
     }
     __syncthreads();
+    if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA of the cluster has started
     for (int j = t; j < J; j += TQ_THREADS) {
         double a = 0;
         for (int w = 0; w < TQ_WARPS; ++w) a = fp_add(a, sums[w * J + j]);  // eight below 0.51p
