@@ -133,9 +133,12 @@ static KInfo kernel_of(const cf_engine* e, int lg, bool wide, long primes) {
 struct Plan {
     int lg, F, d0, nmax, J;
     bool wide = false;  // some prime is 2^50 or above: the kernels for primes below 2^62
+    bool unread = false;  // the primes are not read on the host: a second launch runs those of 2^50 and above
     long primes = MANY_PRIMES;  // primes of the batch, which its geometry follows
     KInfo ki;           // the kernel that runs the batch
     Layout lay;
+    KInfo ki2;          // the kernel of the second launch, and its layout
+    Layout lay2;
     size_t ws_words;
 };
 // The kernel this engine runs for the plan and the workspace layout its geometry needs (the
@@ -144,10 +147,17 @@ static int finalize(cf_engine* e, Plan& pl) {
     const long launch = e && e->max_ctas > 0 ? std::min<long>(pl.primes, e->max_ctas) : pl.primes;
     pl.ki = kernel_of(e, pl.lg, pl.wide, launch);
     if (!pl.ki.fn) return fail(e, CF_ERR_UNSUPPORTED, "no kernel for this transform length");
-    const int nw = pl.ki.threads >= 32 ? pl.ki.threads / 32 : 1;
     // cluster kernels: row sums for the largest cluster, so any cluster size can run the layout
-    pl.lay = make_layout(pl.nmax, pl.F, 1 << pl.lg, pl.J, nw, pl.ki.r, pl.lg > MAX_LG ? MAX_CLUSTER : 1);
+    auto layout = [&](const KInfo& ki) {
+        return make_layout(pl.nmax, pl.F, 1 << pl.lg, pl.J, ki.warps(), ki.r, pl.lg > MAX_LG ? MAX_CLUSTER : 1);
+    };
+    pl.lay = layout(pl.ki);
     pl.ws_words = pl.lay.total;
+    if (pl.unread && !pl.wide) {
+        pl.ki2 = kernel_for(pl.lg, true);
+        pl.lay2 = layout(pl.ki2);
+        pl.ws_words = std::max(pl.ws_words, pl.lay2.total);
+    }
     return CF_OK;
 }
 
@@ -256,6 +266,28 @@ int plan_queries(cf_engine* e, int lg, const KInfo& ki, int J, size_t* smem, int
     return CF_OK;
 }
 
+// One launch of the kernel ki over kp.B primes, one CTA or one cluster each.
+static int launch(cf_engine* e, const KInfo& ki, const KParams& kp, size_t smem, cudaStream_t s) {
+    CF_CUDA(cudaFuncSetAttribute((const void*)ki.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+            "shared memory attribute");
+    if (ki.cluster > 1) {
+        if (ki.cluster > 8)
+            CF_CUDA(cudaFuncSetAttribute((const void*)ki.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                    "cluster size attribute");
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute att[1];
+        att[0].id = cudaLaunchAttributeClusterDimension;
+        att[0].val.clusterDim.x = (unsigned)ki.cluster, att[0].val.clusterDim.y = 1, att[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(kp.B * ki.cluster)), cfg.blockDim = dim3((unsigned)ki.threads);
+        cfg.dynamicSmemBytes = smem, cfg.stream = s, cfg.attrs = att, cfg.numAttrs = 1;
+        CF_CUDA(cudaLaunchKernelEx(&cfg, ki.fn, kp), "cluster kernel launch");
+    } else {
+        ki.fn<<<kp.B, ki.threads, smem, s>>>(kp);
+    }
+    CF_CUDA(cudaGetLastError(), "kernel launch");
+    return CF_OK;
+}
+
 // fixed_ws: use the workspace as it is (a graph capture, where nothing may be allocated)
 // err: the device error word the launch reports to (the engine's unless given)
 static int launch_batch(cf_engine* e, const u64* d_primes, int B, int nmax, int d, int model, int J, const Plan& pl,
@@ -270,8 +302,14 @@ static int launch_batch(cf_engine* e, const u64* d_primes, int B, int nmax, int 
     int JC = 0;
     int rc0 = plan_queries(e, pl.lg, ki, J, &smem, &JC);
     if (rc0) return rc0;
-    CF_CUDA(cudaFuncSetAttribute((const void*)ki.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-            "shared memory attribute");
+    const bool second = pl.unread && !pl.wide;
+    int JC2 = 0;
+    if (second) {
+        int dev = 0, optin = 0;
+        CF_CUDA(cudaGetDevice(&dev), "current device");
+        CF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "shared memory limit");
+        JC2 = pl.ki2.batch_for(J, optin);  // the queries a launch takes are the first kernel's to limit
+    }
     const size_t per_prime = pl.ws_words * 8;
     // chunk: as many primes as the workspace (grown once) holds
     long cap = (long)(e->ws_bytes / per_prime);
@@ -312,24 +350,14 @@ static int launch_batch(cf_engine* e, const u64* d_primes, int B, int nmax, int 
         kp.keep = keep ? keep + (size_t)at * keep_words : nullptr;
         kp.keep_words = keep_words;
         kp.JC = JC;
-        if (ki.cluster > 1) {  // one cluster of ki.cluster CTAs per prime
-            CF_CUDA(cudaFuncSetAttribute((const void*)ki.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                    "shared memory attribute");
-            if (ki.cluster > 8)
-                CF_CUDA(cudaFuncSetAttribute((const void*)ki.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
-                        "cluster size attribute");
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute att[1];
-            att[0].id = cudaLaunchAttributeClusterDimension;
-            att[0].val.clusterDim.x = (unsigned)ki.cluster, att[0].val.clusterDim.y = 1, att[0].val.clusterDim.z = 1;
-            cfg.gridDim = dim3((unsigned)(nb * ki.cluster)), cfg.blockDim = dim3((unsigned)ki.threads);
-            cfg.dynamicSmemBytes = smem, cfg.stream = s, cfg.attrs = att, cfg.numAttrs = 1;
-            CF_CUDA(cudaLaunchKernelEx(&cfg, ki.fn, kp), "cluster kernel launch");
-        } else {
-            ki.fn<<<nb, ki.threads, smem, s>>>(kp);
-        }
-        CF_CUDA(cudaGetLastError(), "kernel launch");
+        rc0 = launch(e, ki, kp, smem, s);
+        if (rc0) return rc0;
         ++e->launches;
+        if (second) {
+            kp.lay = pl.lay2, kp.JC = JC2, kp.p_lo = 1ull << 50;
+            rc0 = launch(e, pl.ki2, kp, pl.ki2.smem_for(JC2), s);
+            if (rc0) return rc0;
+        }
     }
     return CF_OK;
 }
@@ -682,6 +710,7 @@ int cf_residues_async(cf_engine* e, const uint64_t* d_primes, int B, int nmax, i
     if (rc) return rc;
     if (B == 0) return CF_OK;
     pl.wide = e->prime_bits > 50;
+    pl.unread = true;
     pl.primes = B;
     rc = finalize(e, pl);
     if (rc) return rc;
@@ -764,6 +793,7 @@ int cf_batch_graph_create(cf_engine* e, const uint64_t* d_primes, int B, int nma
     int rc = plan(e, nmax, d, model, qn, qM, J, pl);
     if (rc) return rc;
     pl.wide = e->prime_bits > 50;
+    pl.unread = true;
     pl.primes = B;
     rc = finalize(e, pl);
     if (rc) return rc;

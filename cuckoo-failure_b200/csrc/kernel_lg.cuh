@@ -161,11 +161,22 @@ struct Geometry {
                                          : 1;
 };
 constexpr int few_per_sm(int lg) { return lg == 12 ? 1 : lg >= 8 && lg <= 10 ? 2 : 0; }
+// Does this launch leave prime P alone?  The double-precision kernels compute nothing for a prime of
+// 2^50 or above; where the host has not read the primes (cf_residues_async, batch graphs), a launch of
+// the integer kernels follows for those, which leaves the primes below kp.p_lo = 2^50 alone.  A second
+// launch rather than a branch: with the integer path as a function of these kernels their registers
+// shifted, and they ran up to 5 % slower (n = 1500, 148 primes: 17.4 -> 18.2 ms); launched, it adds
+// 2.4 to 4 us to a call (n = 24, one prime: 114.7 -> 117.0 us).
+template <bool W>
+__device__ __forceinline__ bool not_ours(const KParams& kp, u64 P) {
+    return W ? P < kp.p_lo : P >> 50 != 0;
+}
 // MB: resident CTAs per SM the variant is compiled for (its register cap).
 template <int LG, int R, bool W, int MB>
 __global__ void __launch_bounds__(Geo<LG, R>::T, MB) k_suffix(KParams kp) {
     typedef Geo<LG, R> G;
     extern __shared__ __align__(16) u64 smem[];
+    if (not_ours<W>(kp, kp.primes[blockIdx.x])) return;
     DevExec<G> ex;
     PrimeRun<G, DevExec<G>, W> pr(ex, kp, (int)blockIdx.x, smem);
     pr.run();
@@ -253,6 +264,7 @@ template <int LG, int R, int LC, bool W>
 __global__ void __launch_bounds__(Geo<LG, R, LC>::CT, 1) k_suffix_cl(KParams kp) {
     typedef Geo<LG, R, LC> G;
     extern __shared__ __align__(16) u64 smem[];
+    if (not_ours<W>(kp, kp.primes[blockIdx.x >> LC])) return;  // all CTAs of the cluster
     DevExec<G> ex;
     PrimeRun<G, DevExec<G>, W> pr(ex, kp, (int)blockIdx.x >> LC, smem);
     pr.run();

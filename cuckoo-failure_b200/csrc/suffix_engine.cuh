@@ -329,6 +329,7 @@ struct KParams {
     u64* keep = nullptr;  // resident tables [B][keep_words] (serving builds), or null
     size_t keep_words = 0;
     int JC = 0;  // queries whose partial sums shared memory holds at a time (0: all J)
+    u64 p_lo = 0;  // an integer-kernel launch leaves primes below it alone (another launch's)
 };
 
 // Error codes recorded in *err by the kernel.

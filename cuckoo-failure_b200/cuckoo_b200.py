@@ -228,7 +228,8 @@ class Engine:
         return out
 
     def residues_async(self, d_primes_ptr, B, nmax, d, queries, d_out_ptr, stream_ptr=None, model=MODEL_SUBSET):
-        """Device-pointer variant (e.g. torch tensors' data_ptr()); enqueued on stream_ptr."""
+        """Device-pointer variant (e.g. torch tensors' data_ptr()); enqueued on stream_ptr.  The primes
+        are not read on the host: any below 2^62 may be among them (set_prime_bits)."""
         qn, qM = _queries(queries)
         rc = lib().cf_residues_async(self._h, ctypes.c_void_p(d_primes_ptr), B, nmax, d, model,
                                      qn.ctypes.data_as(_intp), qM.ctypes.data_as(_intp), len(qn),
@@ -274,6 +275,12 @@ class Engine:
     def set_transform_lg(self, lg):
         """Transforms of at least 2^lg entries (0: the reference's length); residues do not change."""
         self._check(lib().cf_engine_set_transform_lg(self._h, lg))
+
+    def set_prime_bits(self, bits):
+        """For calls whose primes are on the device: 50 (the default) runs primes below 2^50 in double
+        precision and passes once more over the batch for those from 2^50 to 2^62; 62 runs all of them on
+        the kernels for primes below 2^62."""
+        self._check(lib().cf_engine_set_prime_bits(self._h, bits))
 
     def set_max_ctas(self, n):
         """At most n primes (CTAs) per launch of this engine's batches (0: no cap)."""

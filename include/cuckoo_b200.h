@@ -81,7 +81,10 @@ int cf_residues(cf_engine* e, const uint64_t* primes, int B, int nmax, int d, in
 
 /* Same computation with the primes and residues in device memory, enqueued on `stream`
  * (a cudaStream_t; NULL is the CUDA default stream); returns without waiting.  The primes are
- * not read on the host: they must lie below 2^50 unless cf_engine_set_prime_bits(e, 62). */
+ * not read on the host and not checked, but any below 2^62 may be among them: a launch of the kernels
+ * for primes below 2^50, which passes over the others, is followed by one of the kernels for primes
+ * below 2^62, which ends at once where there are none.  cf_engine_set_prime_bits(e, 62) runs the
+ * latter alone, for all primes (50, the default: both). */
 int cf_engine_set_prime_bits(cf_engine* e, int bits);
 int cf_residues_async(cf_engine* e, const uint64_t* d_primes, int B, int nmax, int d, int model, const int* qn,
                       const int* qM, int J, uint64_t* d_residues, void* stream);
@@ -98,7 +101,8 @@ long cf_max_batch(cf_engine* e, int nmax, int Mmax, int J);
  * No counterpart in the reference, whose batch is bounded by memory only (:743-780). */
 long cf_resident_primes(cf_engine* e, int nmax, int Mmax, int J);
 
-/* Kernel launches issued by the last cf_residues / cf_residues_async call. */
+/* Kernel launches issued by the last cf_residues / cf_residues_async call, not counting the pass of
+ * cf_residues_async over primes of 2^50 and above. */
 long cf_last_launches(const cf_engine* e);
 
 /* ---- graph-captured batches (no counterpart in the reference) ----
@@ -118,7 +122,8 @@ int cf_batch_graph_launch(cf_batch_graph* g, void* stream);
 /* Wait for the work on `stream` and report the device-side checks of the graph's last replay:
  * CF_OK, or CF_ERR_DEVICE (e.g. a prime without a root of unity of order L). */
 int cf_batch_graph_status(cf_batch_graph* g, void* stream);
-/* Kernel launches (persistent-kernel nodes) in one replay. */
+/* Kernel launches (persistent-kernel nodes) in one replay, not counting the pass over primes of 2^50
+ * and above (cf_residues_async). */
 long cf_batch_graph_launches(const cf_batch_graph* g);
 void cf_batch_graph_destroy(cf_batch_graph* g);
 
