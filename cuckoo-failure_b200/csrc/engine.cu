@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -579,29 +580,33 @@ static int tables_query(cf_engine* e, const cf_tables* t, const int* qn, const i
         if (t->model == CF_MODEL_SUBSET && t->d > qM[j]) return fail(e, CF_ERR_ARG, "subset model needs d <= M");
     }
     const int sms = sm_count();
-    std::vector<int> order;
     for (int j0 = 0; j0 < J; j0 += TQ_MAXJ) {
         TQParams tp;
         tp.primes = t->d_primes;
         tp.B = t->B, tp.n = t->n, tp.F = t->F, tp.d = t->d, tp.d0 = t->d0, tp.model = t->model;
         tp.J = std::min(TQ_MAXJ, J - j0);
-        order.resize((size_t)tp.J);
-        for (int j = 0; j < tp.J; ++j) order[(size_t)j] = j0 + j;
-        std::sort(order.begin(), order.end(), [&](int a, int b) { return qn[a] > qn[b]; });  // largest tables first
-        for (int j = 0; j < tp.J; ++j) tp.qn[j] = qn[order[(size_t)j]], tp.qM[j] = qM[order[(size_t)j]], tp.qi[j] = (short)(order[(size_t)j] - j0);
+        u32 order[TQ_MAXJ];  // size and place, largest tables first
+        for (int j = 0; j < tp.J; ++j) order[j] = (u32)qn[j0 + j] << 8 | (u32)j;
+        std::sort(order, order + tp.J, std::greater<u32>());
         tp.keep = t->keep;
         tp.keep_words = t->keep_words;
         tp.out = d_out + j0;
         tp.out_stride = (size_t)J;
-        tp.S = tq_ctas(t->B, tp.qn[0], sms);
-        const size_t smem = tq_smem_bytes(tp.J);
+        const TQSplit split = tq_split(t->B, tp.J, (int)(order[0] >> 8), sms);
+        tp.S = split.S, tp.G = split.G, tp.W = split.W;
+        for (int g = 0, k = 0; g < tp.G; ++g)  // group g: every G-th of them
+            for (int j = g; j < tp.J; j += tp.G, ++k) {
+                const int i = (int)(order[j] & 255);
+                tp.qn[k] = qn[j0 + i], tp.qM[k] = qM[j0 + i], tp.qi[k] = (short)i;
+            }
+        const size_t smem = tq_smem_bytes((tp.J + tp.G - 1) / tp.G);
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute att[1];
         att[0].id = cudaLaunchAttributeClusterDimension;
         att[0].val.clusterDim.x = (unsigned)tp.S, att[0].val.clusterDim.y = 1, att[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3((unsigned)(t->B * tp.S)), cfg.blockDim = dim3(TQ_THREADS), cfg.dynamicSmemBytes = smem;
-        cfg.stream = s, cfg.attrs = att, cfg.numAttrs = 1;
-        CF_CUDA(cudaLaunchKernelEx(&cfg, k_table_query, tp), "query launch");
+        cfg.gridDim = dim3((unsigned)(t->B * tp.G * tp.S)), cfg.blockDim = dim3(TQ_THREADS), cfg.dynamicSmemBytes = smem;
+        cfg.stream = s, cfg.attrs = att, cfg.numAttrs = tp.S > 1 ? 1 : 0;
+        CF_CUDA(cudaLaunchKernelEx(&cfg, tp.W * tp.G >= tp.J ? k_table_query<true> : k_table_query<false>, tp), "query launch");
         ++e->launches;
     }
     return CF_OK;

@@ -19,15 +19,17 @@
 #include <cuda_runtime.h>
 
 #include "suffix_engine.cuh"
+#include "table_split.hpp"
 
 namespace cfb {
 
 // Queries per launch: their sizes travel in the kernel parameters (no staging buffer, so launches
 // on several streams never share one).
-constexpr int TQ_MAXJ = 256;
+constexpr int TQ_MAXJ = 256;  // (the host sorts by size << 8 | place)
 struct TQParams {
     const u64* primes;  // [B]
-    int B, n, F, d, d0, model, J, S;  // S: CTAs per prime
+    int B, n, F, d, d0, model, J;
+    int S, G, W;        // the launch's split (tq_split)
     const u64* keep;    // [B][keep_words]
     size_t keep_words;
     u64* out;           // residue of prime b, query jq at out[b * out_stride + jq]
@@ -37,36 +39,23 @@ struct TQParams {
     short qi[TQ_MAXJ];  // the query's place in out
 };
 
-constexpr int TQ_THREADS = 256, TQ_WARPS = TQ_THREADS / 32, TQ_PER_SM = 2;
-constexpr int TQ_ROWS = 16, TQ_K = 8, TQ_COLS = 32 * TQ_K;  // a warp's tile: rows, columns per lane, columns
-constexpr int TQ_CLUSTER = 4;                               // CTAs per prime at most
-// Shared memory: per query Q and the warps' sums, and (read from the first CTA) the CTAs' sums.
-inline size_t tq_smem_bytes(int J) { return 8 * (size_t)J * (1 + TQ_WARPS + TQ_CLUSTER); }
-// CTAs per prime: the number up to TQ_CLUSTER whose waves of resident CTAs leave the least idle (the
-// CTAs' shares are equal, so a launch lasts waves / S), with a block of rows for every warp.
-// Four at most: beside a plain rebuild that fills 96 SMs, clusters of eight find fewer places in what
-// each GPC has left (served requests with n in 513 .. 2048: p50 10.6 ms, p99 44; with four 5.9 and 28).
-inline int tq_ctas(int B, int nmax, int sms) {
-    const long cap = (long)TQ_PER_SM * (sms > 0 ? sms : 1);
-    int S = 1;
-    for (int c = 2; c <= TQ_CLUSTER && nmax >= TQ_ROWS * TQ_WARPS * c / 2; ++c)
-        if (((long)B * c + cap - 1) / cap * S < ((long)B * S + cap - 1) / cap * c) S = c;
-    return S;
-}
+// Shared memory: per query of a group Q and the warps' sums, and (read from the first CTA) the CTAs' sums.
+inline size_t tq_smem_bytes(int Jg) { return 8 * (size_t)Jg * (1 + TQ_WARPS + TQ_CLUSTER); }
 
 // a whole number below 2^52 as a double
 __device__ __forceinline__ double tq_double(u64 v) { return __dadd_rn(__longlong_as_double((long long)(v | 0x4330000000000000ull)), -4503599627370496.0); }
 __device__ __forceinline__ double tq_load(const u64* p) { return tq_double(__ldg(p)); }  // resident tables: another launch's writes
 
-// One tile, rows q0 .. q0 + TQ_ROWS - 1 and columns w0 .. w0 + TQ_COLS - 1, for queries j0 .. j0 + NJ - 1:
-// its part of their sums is added to sums[].
+// One tile, rows q0 .. q0 + TQ_ROWS - 1 and columns w0 .. w0 + TQ_COLS - 1, for the group's queries
+// j0 .. j0 + NJ - 1 (query j of the group is g0 + j of the launch): its part of their sums is added to sums[].
 template <int NJ>
 __device__ __forceinline__ void tq_tile(const TQParams& tp, const KeepLayout& kl, const u64* base, const FpMod& m, int q0, int w0,
-                                        int j0, const double* Qs, double* sums) {
+                                        int g0, int j0, const double* Qs, double* sums) {
+    auto at = [&](int j) { return g0 + j; };
     const int lane = threadIdx.x & 31, d0 = tp.d0;
     const u64* inv = base + kl.inv;
     const u64* tri = base + kl.tri + w0 + lane;
-    const int qe = min(q0 + TQ_ROWS - 1, tp.qn[j0]);  // the last row a query needs (sizes descend)
+    const int qe = min(q0 + TQ_ROWS - 1, tp.qn[at(j0)]);  // the last row a query needs (sizes descend)
     u64 next[TQ_K];
     auto get = [&](int q) {
         const u64* row = tri + tri_off((size_t)q);
@@ -80,7 +69,7 @@ __device__ __forceinline__ void tq_tile(const TQParams& tp, const KeepLayout& kl
     // lane r + TQ_ROWS j computes F of row q0 + r for query j0 + j (zero past the query's size)
     double F = 0;
     {
-        const int j = NJ > 1 ? j0 + lane / TQ_ROWS : j0, q = q0 + lane % TQ_ROWS, nj = tp.qn[j], Mj = tp.qM[j];
+        const int j = NJ > 1 ? j0 + lane / TQ_ROWS : j0, q = q0 + lane % TQ_ROWS, nj = tp.qn[at(j)], Mj = tp.qM[at(j)];
         if (q <= nj) {
             F = fp_mulmod(tq_load(inv + 2 * (size_t)q), tq_load(base + kl.ifact + 2 * (size_t)(nj - q)), m);
             F = fp_mulmod(F, tq_load(base + kl.ifact + 2 * (size_t)(Mj - q)), m);
@@ -112,7 +101,7 @@ __device__ __forceinline__ void tq_tile(const TQParams& tp, const KeepLayout& kl
     }
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-        const int Mj = tp.qM[j0 + j];
+        const int Mj = tp.qM[at(j0 + j)];
         double y = 0;
 #pragma unroll
         for (int k = 0; k < TQ_K; ++k) {
@@ -131,10 +120,14 @@ __device__ __forceinline__ void tq_tile(const TQParams& tp, const KeepLayout& kl
     __syncwarp();
 }
 
-// S CTAs (a cluster) per prime: CTA b S + s is CTA s of prime b.
-__global__ void __launch_bounds__(TQ_THREADS, TQ_PER_SM) k_table_query(TQParams tp) {
+// A cluster of S CTAs per prime and group: CTA (b G + g) S + s is CTA s of prime b and group g.  ALL: a
+// warp takes all the group's queries of a tile (W >= J; one kernel for both ways of dealing ran 1.4 % slower).
+template <bool ALL>
+__global__ void __launch_bounds__(TQ_THREADS, TQ_PER_SM) k_table_query(const __grid_constant__ TQParams tp) {
     extern __shared__ __align__(16) double tq_sm[];
-    const int S = tp.S, b = blockIdx.x / S, s = blockIdx.x % S, J = tp.J;
+    const int S = tp.S, G = tp.G, s = blockIdx.x % S, g = blockIdx.x / S % G, b = blockIdx.x / S / G;
+    const int J = tp.J / G + (g < tp.J % G), g0 = tp.J / G * g + min(g, tp.J % G);  // the group's queries
+    auto at = [&](int j) { return g0 + j; };
     const int t = threadIdx.x, warp = t >> 5;
     if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // waited for before the first remote store
     double* Qs = tq_sm;                    // [J] candidate sets per item
@@ -147,25 +140,36 @@ __global__ void __launch_bounds__(TQ_THREADS, TQ_PER_SM) k_table_query(TQParams 
     const u64* base = tp.keep + (size_t)b * tp.keep_words;
     const u64 *fact = base + kl.fact, *ifact = base + kl.ifact;
     for (int j = t; j < J; j += TQ_THREADS) {
-        const int Mj = tp.qM[j];
+        const int Mj = tp.qM[at(j)];
         Qs[j] = tp.model == MODEL_REPLACEMENT
                     ? fp_pow((double)Mj, (u64)tp.d, m)
                     : fp_mulmod(fp_mulmod(tq_load(fact + 2 * (size_t)Mj), tq_load(ifact + 2 * (size_t)tp.d), m), tq_load(ifact + 2 * (size_t)(Mj - tp.d)), m);
     }
     for (int k = t; k < TQ_WARPS * J; k += TQ_THREADS) sums[k] = 0;
     __syncthreads();
-    // tiles, the last rows first, dealt to the prime's warps in turn
+    // (tile, W queries) units, the last rows first, dealt to the cluster's warps in turn
     const int nw = S * TQ_WARPS, me = warp * S + s;
-    int at = 0;
-    for (int blk = (tp.qn[0] - 1) / TQ_ROWS; blk >= 0; --blk) {
-        const int q0 = 1 + TQ_ROWS * blk, tiles = (min(q0 + TQ_ROWS - 1, tp.qn[0]) + TQ_COLS - 1) / TQ_COLS;  // columns 0 .. q0 + TQ_ROWS - 2
+    int dealt = 0, jn = 0;  // jn: queries that have row q0
+    for (int blk = (tp.qn[g0] - 1) / TQ_ROWS; blk >= 0; --blk) {
+        const int q0 = 1 + TQ_ROWS * blk, tiles = (min(q0 + TQ_ROWS - 1, tp.qn[g0]) + TQ_COLS - 1) / TQ_COLS;  // columns 0 .. q0 + TQ_ROWS - 2
         if (q0 + TQ_ROWS - 1 <= tp.d0) break;
-        for (int c = (me - at % nw + nw) % nw; c < tiles; c += nw)
-            for (int j = 0; j < J && tp.qn[j] >= q0;) {
-                if (j + 1 < J && tp.qn[j + 1] >= q0) tq_tile<2>(tp, kl, base, m, q0, c * TQ_COLS, j, Qs, sums + warp * J), j += 2;
-                else tq_tile<1>(tp, kl, base, m, q0, c * TQ_COLS, j, Qs, sums + warp * J), j += 1;
+        if constexpr (ALL) {
+            for (int c = (me - dealt % nw + nw) % nw; c < tiles; c += nw)
+                for (int j = 0; j < J && tp.qn[g0 + j] >= q0;) {
+                    if (j + 1 < J && tp.qn[g0 + j + 1] >= q0) tq_tile<2>(tp, kl, base, m, q0, c * TQ_COLS, g0, j, Qs, sums + warp * J), j += 2;
+                    else tq_tile<1>(tp, kl, base, m, q0, c * TQ_COLS, g0, j, Qs, sums + warp * J), j += 1;
+                }
+            dealt += tiles;
+        } else {
+            while (jn < J && tp.qn[g0 + jn] >= q0) ++jn;
+            const int parts = (jn + tp.W - 1) / tp.W, units = tiles * parts;
+            for (int u = (me - dealt % nw + nw) % nw; u < units; u += nw) {
+                const int c = u / parts, j = (u - c * parts) * tp.W;
+                if (tp.W > 1 && j + 1 < jn) tq_tile<2>(tp, kl, base, m, q0, c * TQ_COLS, g0, j, Qs, sums + warp * J);
+                else tq_tile<1>(tp, kl, base, m, q0, c * TQ_COLS, g0, j, Qs, sums + warp * J);
             }
-        at += tiles;
+            dealt += units;
+        }
     }
     __syncthreads();
     if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA of the cluster has started
@@ -189,9 +193,9 @@ __global__ void __launch_bounds__(TQ_THREADS, TQ_PER_SM) k_table_query(TQParams 
     for (int j = t; j < J; j += TQ_THREADS) {  // N_bad = M! n! sum of the terms
         double a = 0;
         for (int c = 0; c < S; ++c) a = fp_add(a, all[c * J + j]);
-        a = fp_mulmod(fp_red(a, m), tq_load(fact + 2 * (size_t)tp.qn[j]), m);
-        a = fp_mulmod(a, tq_load(fact + 2 * (size_t)tp.qM[j]), m);
-        tp.out[(size_t)b * tp.out_stride + tp.qi[j]] = fp_canon(a, m);
+        a = fp_mulmod(fp_red(a, m), tq_load(fact + 2 * (size_t)tp.qn[at(j)]), m);
+        a = fp_mulmod(a, tq_load(fact + 2 * (size_t)tp.qM[at(j)]), m);
+        tp.out[(size_t)b * tp.out_stride + tp.qi[at(j)]] = fp_canon(a, m);
     }
 }
 
