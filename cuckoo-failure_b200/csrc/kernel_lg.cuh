@@ -133,12 +133,16 @@ struct DevExec {
 //   2^9:  4 x 128 at 296 primes 3.7 against 4.9, at 360 6.8 against 5.8 (n = 500): 2 per SM
 //   2^8:  2 x 128 at 296 primes 1.33 against 1.42, at 360 2.26 against 1.47 (n = 200): 2 per SM
 //
-// Primes below 2^62 (64-bit integers), one CTA's registers uncapped (ms per launch, n = 2^LG or the
+// Primes below 2^62 (64-bit integers), registers uncapped above 2^8 (ms per launch, n = 2^LG or the
 // stated n; in front the geometries with half to an eighth of the threads that were the default):
 //   2^13: 16 x 512 941, 8 x 1024 762 (148 primes)     2^12: 16 x 256 269, 8 x 512 179, 4 x 1024 200 (148)
 //   2^11: 16 x 128 126, 8 x 256 72, 4 x 512 51 (148); 271, 288, 204 (592)
 //   2^10: 32 x 32 126, 8 x 128 32, 4 x 256 14.4 (n = 1000, 148); 499, 270, 229 (2368)
 //   2^9:  16 x 32 30, 4 x 128 6.2, 2 x 256 5.5 (148); 34, 17, 21 (592)   2^8: 8 x 32 7.2, 4 x 64 2.9 (148); 8.1, 3.8 (592)
+// Up to 2^8 the registers are capped at 128 (no spills), for 16 CTAs of a warp or 8 of two on an SM;
+// uncapped they took 151 to 190 and fewer fitted (ms, 2368 primes, one query; in front the form with
+// half the threads at 2^7 and 2^8 and all 121 to 238, then uncapped, then capped): n = 40 1.02, 1.24, 1.01; n = 64 1.48, 1.91, 1.48;
+// n = 128 (1184 primes) 2.42, 2.85, 2.17; n = 200 14.07 with nine queries, 14.87, 12.54.
 template <int LG, bool W, bool FEW = false>
 struct Geometry {
     static constexpr int R = W          ? (LG == 14 ? 4 : LG >= 12 ? 3 : LG >= 10 ? 2 : LG >= 8 ? 2 : 1)
@@ -150,7 +154,7 @@ struct Geometry {
                              : LG == 9  ? (FEW ? 2 : 3)
                              : LG == 8  ? (FEW ? 1 : 2)
                                         : 1;
-    static constexpr int MB = W          ? 1
+    static constexpr int MB = W          ? (LG <= 6 ? 16 : LG <= 8 ? 8 : 1)
                               : LG >= 13 ? 1
                               : LG == 12 ? (FEW ? 1 : 2)
                               : LG == 11 ? 3

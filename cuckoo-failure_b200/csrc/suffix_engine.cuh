@@ -524,7 +524,8 @@ struct PrimeBase {
         }
     }
     CF_HD void fold_last(int q) {
-        if (kp.J > 0) fold_queries(q, (kp.J - 1) / query_batch() * query_batch(), kp.J);
+        const int jc = query_batch();
+        if (kp.J > 0) fold_queries(q, jc == kp.J ? 0 : (kp.J - 1) / jc * jc, kp.J);  // no division where one batch holds all
     }
 
     // The full tile's columns v0 .. v0 + 15 into row storage, the rows r = t + jT of the warp's threads (rows of
@@ -567,7 +568,9 @@ struct PrimeBase {
     // is complete after the barrier.  keep(v0, v): copies the tile's columns of a serving build.
     template <class F>
     CF_HD void end_step(int v, F&& keep) {
-        constexpr int FL = CT >= 1024 ? 8 : TILE;  // columns of S and of V in flight per thread
+        // columns of S and of V in flight per thread: fewer where registers bound the threads (1024 of them,
+        // or a warp or less to a CTA, where 16 columns took 160 registers and four CTAs fewer fit an SM)
+        constexpr int FL = CT >= 1024 ? 8 : CT <= 32 ? 4 : TILE;
         const int n = kp.n, d0 = kp.d0;
         const int v0 = tile_v0(v);
         if (v - v0 == TILE - 1 || v == n - 1) {  // move the tile's columns v0 .. v into the rows
