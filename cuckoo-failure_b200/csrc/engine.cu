@@ -18,12 +18,13 @@
 
 using namespace cfb;
 
-static int sm_count() {  // of the current device
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+static int sm_count(int device = -1) {  // of a device, the current one if negative
+    int sms = 0;
+    if (device < 0 && cudaGetDevice(&device) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
     return sms;
 }
-KInfo kernel_for(int lg, bool wide, long primes) {
+KInfo kernel_for(int lg, bool wide, long primes, int device) {
     if (wide) switch (lg) {
             case 4: return cf_kinfo_lg4_w();
             case 5: return cf_kinfo_lg5_w();
@@ -40,7 +41,7 @@ KInfo kernel_for(int lg, bool wide, long primes) {
             case 16: return cf_kinfo_lg16_c8_w();
             default: return KInfo{nullptr, 0, 0, 0};
         }
-    if (few_per_sm(lg) > 0 && primes < MANY_PRIMES && primes <= (long)few_per_sm(lg) * sm_count()) switch (lg) {
+    if (few_per_sm(lg) > 0 && primes < MANY_PRIMES && primes <= (long)few_per_sm(lg) * sm_count(device)) switch (lg) {
             case 8: return cf_kinfo_lg8_few();
             case 9: return cf_kinfo_lg9_few();
             case 10: return cf_kinfo_lg10_few();
@@ -128,7 +129,7 @@ static KInfo kernel_of(const cf_engine* e, int lg, bool wide, long primes) {
         KInfo v[MAX_VARIANTS];
         if (e->tuned[lg] < variants_for(lg, v, MAX_VARIANTS)) return v[e->tuned[lg]];
     }
-    return kernel_for(lg, wide, primes);
+    return kernel_for(lg, wide, primes, e ? e->device : -1);
 }
 
 struct Plan {

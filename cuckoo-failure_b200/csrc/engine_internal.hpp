@@ -38,9 +38,9 @@ cfb::KInfo cf_kinfo_lg10_few();
 cfb::KInfo cf_kinfo_lg12_few();
 // The default kernel for transform length 2^lg: primes below 2^50, or (wide) below 2^62; below 2^50 the
 // geometry for few primes when a launch has no more than `primes` of them (Geometry in
-// kernel_lg.cuh; engine.cu).
+// kernel_lg.cuh; engine.cu) for the SMs of `device`, the current one if negative.
 constexpr long MANY_PRIMES = 1l << 40;
-cfb::KInfo kernel_for(int lg, bool wide = false, long primes = MANY_PRIMES);
+cfb::KInfo kernel_for(int lg, bool wide = false, long primes = MANY_PRIMES, int device = -1);
 cfb::KInfo cf_kinfo_lg15_c4();
 cfb::KInfo cf_kinfo_lg15_c8();
 cfb::KInfo cf_kinfo_lg15_c4_e8();
