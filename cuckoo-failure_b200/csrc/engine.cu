@@ -123,7 +123,8 @@ static int variants_for(int lg, KInfo* v, int cap) {
     }
 }
 constexpr int MAX_VARIANTS = 8;
-// The kernel an engine runs: for primes below 2^50 the geometry it was tuned to, else the default.
+// The kernel an engine runs: for primes below 2^50 the geometry it was tuned to, else (index 0) the default,
+// which follows the number of primes.
 static KInfo kernel_of(const cf_engine* e, int lg, bool wide, long primes) {
     if (!wide && e && lg >= 0 && lg <= MAX_LG && e->tuned[lg] > 0) {
         KInfo v[MAX_VARIANTS];
@@ -877,6 +878,17 @@ int cf_tune_variants(int lg, int* log2_entries, int* threads, int* ctas_per_sm, 
         if (ctas_per_sm) ctas_per_sm[i] = v[i].mb;
     }
     return k;
+}
+
+int cf_tune_geometry(const cf_engine* e, int lg, int variant, int primes, int* log2_entries, int* threads, int* ctas_per_sm) {
+    if (!e || lg < 0 || lg > MAX_LG_CLUSTER || variant < 0 || primes < 1) return CF_ERR_ARG;
+    KInfo v[MAX_VARIANTS];
+    if (variant >= (lg > MAX_LG ? cluster_variants(lg, v) : variants_for(lg, v, MAX_VARIANTS))) return CF_ERR_ARG;
+    if (variant == 0 && lg <= MAX_LG) v[0] = kernel_for(lg, false, e->max_ctas > 0 ? std::min(primes, e->max_ctas) : primes, e->device);
+    if (log2_entries) *log2_entries = v[variant].r;
+    if (threads) *threads = v[variant].threads;
+    if (ctas_per_sm) *ctas_per_sm = v[variant].mb;
+    return CF_OK;
 }
 
 int cf_tune_set(cf_engine* e, int lg, int variant) {

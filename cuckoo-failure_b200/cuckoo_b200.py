@@ -75,6 +75,8 @@ def lib():
         L.cf_resident_primes.restype = ctypes.c_long
         L.cf_tune_variants.argtypes = [ctypes.c_int, _intp, _intp, _intp, ctypes.c_int]
         L.cf_tune_variants.restype = ctypes.c_int
+        L.cf_tune_geometry.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, _intp, _intp, _intp]
+        L.cf_tune_geometry.restype = ctypes.c_int
         L.cf_autotune.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                   ctypes.POINTER(ctypes.c_double), ctypes.c_int, _intp]
         L.cf_autotune.restype = ctypes.c_int
@@ -169,7 +171,7 @@ def lib_primes(n, M, d, model=MODEL_SUBSET):
 
 
 def tune_variants(lg):
-    """The compiled geometries for transform length 2^lg, the default first:
+    """The compiled geometries for transform length 2^lg, the default (as batches of many primes run it) first:
     [{"entries_per_thread": 2^r, "threads": T, "ctas_per_sm": k}]."""
     r, t, m = (np.zeros(8, dtype=np.int32) for _ in range(3))
     k = int(lib().cf_tune_variants(lg, r.ctypes.data_as(_intp), t.ctypes.data_as(_intp), m.ctypes.data_as(_intp), 8))
@@ -254,13 +256,23 @@ class Engine:
 
     def autotune(self, nmax, Mmax, d, B):
         """Time every compiled geometry for nmax's transform length on B primes (cf_autotune) and
-        keep the fastest: returns {"lg", "chosen", "rates" (primes/s per geometry), "variants"}."""
+        keep the fastest: returns {"lg", "chosen", "rates" (primes/s per geometry), "variants" (the
+        geometries as they ran)}."""
         lg = transform_length(nmax).bit_length() - 1
         rates = (ctypes.c_double * 8)()
         chosen = ctypes.c_int(0)
         self._check(lib().cf_autotune(self._h, nmax, Mmax, d, B, rates, 8, ctypes.byref(chosen)))
-        vs = tune_variants(lg)
+        vs = self.tune_variants(lg, B)
         return {"lg": lg, "chosen": chosen.value, "rates": [rates[i] for i in range(len(vs))], "variants": vs}
+
+    def tune_variants(self, lg, B):
+        """tune_variants(lg) as launches of B primes on this engine run them: the default's geometry follows
+        the number of primes."""
+        out, r = [], [ctypes.c_int(0) for _ in range(3)]
+        for i in range(len(tune_variants(lg))):
+            self._check(lib().cf_tune_geometry(self._h, lg, i, B, *(ctypes.byref(x) for x in r)))
+            out.append({"entries_per_thread": 1 << r[0].value, "threads": r[1].value, "ctas_per_sm": r[2].value})
+        return out
 
     def tune_set(self, lg, variant):
         self._check(lib().cf_tune_set(self._h, lg, variant))

@@ -43,7 +43,7 @@ def tuned(engine, nmax, Mmax, d, B, cache=DEFAULT_CACHE, device_name=None):
         except (OSError, ValueError):
             data = {}
     rec = data.get(key)
-    if rec is not None and rec.get("variants") == cb.tune_variants(lg):
+    if rec is not None and rec.get("variants") == engine.tune_variants(lg, B):
         engine.tune_set(lg, rec["chosen"])
         return {**rec, "source": "cache"}
     rec = engine.autotune(nmax, Mmax, d, B)

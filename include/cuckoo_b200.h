@@ -136,6 +136,9 @@ void cf_batch_graph_destroy(cf_batch_graph* g);
  * Mmax), d) through cf_residues, checks that all give the same residues, and makes the fastest
  * the engine's choice for that length (rates[i]: primes per second of geometry i, *chosen: the
  * index).  cf_tune_set / cf_tune_get pin or read the choice (e.g. from a cache of earlier runs).
+ * Index 0 is the default: at 2^8, 2^9, 2^10 and 2^12 a launch of few primes runs it with more threads per
+ * prime than cf_tune_variants says; cf_tune_geometry describes geometry i as a launch of that many
+ * primes on the engine runs it.
  * Primes below 2^62 always use the default geometry.
  * Transform lengths 2^15 and 2^16 (nmax > 16384) run one prime per thread-block cluster: their
  * variants are the cluster geometries compiled (threads = CTA size, 2^log2_entries entries each,
@@ -143,6 +146,7 @@ void cf_batch_graph_destroy(cf_batch_graph* g);
  * the fastest measured on B200; cf_tune_set(e, lg, i) pins variant i (-1: the default again),
  * cf_tune_get returns the pinned index or -1, and cf_autotune times them like the others. */
 int cf_tune_variants(int lg, int* log2_entries, int* threads, int* ctas_per_sm, int cap);
+int cf_tune_geometry(const cf_engine* e, int lg, int variant, int primes, int* log2_entries, int* threads, int* ctas_per_sm);
 int cf_autotune(cf_engine* e, int nmax, int Mmax, int d, int B, double* rates, int cap, int* chosen);
 int cf_tune_set(cf_engine* e, int lg, int variant);
 int cf_tune_get(const cf_engine* e, int lg);

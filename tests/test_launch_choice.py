@@ -27,3 +27,21 @@ def test_geometry_follows_the_engines_device(fake, other):
                     assert dev == 1 - other and grid == 100
                     threads.append(block)
                 assert threads[0] == threads[1], n
+
+
+@pytest.mark.parametrize("n", [200, 500, 1000, 4096])
+@pytest.mark.parametrize("B,cap", [(100, 0), (148, 0), (296, 0), (592, 0), (592, 100)])
+def test_autotune_record_describes_what_ran(fake, n, B, cap):
+    """The geometries of an autotuning record are those its launches had, the default's among them."""
+    with fd.on(fake) as L:
+        L.fake_set_sms(0, 148)
+        with cb.Engine(0) as eng:
+            assert L.cf_engine_set_max_ctas(eng._h, cap) == 0
+            fd.launches(L)
+            rec = eng.autotune(n, 2 * n, 3, B)
+            ran = fd.launches(L)
+            per = len(ran) // len(rec["variants"])
+            assert [v["threads"] for v in rec["variants"]] == [block for _, _, block, _ in ran[::per]]
+            eng.tune_set(rec["lg"], 0)
+            eng.residues(cb.prime_range(0, B), n, 3, [(n, 2 * n)])
+            assert fd.launches(L)[0][2] == rec["variants"][0]["threads"]
