@@ -36,10 +36,6 @@ UNIT = "prime-residues/s"
 # Operations per modular multiplication by prime bits (fixed accounting model): below 2^50 a product is six
 # double-precision operations and a butterfly adds two; below 2^62 a Shoup product is 20 INT32 multiplies.
 OPS_PER_MM = {50: (8, "fp64", "Top/s (FP64 instructions' lanes)"), 62: (20, "int32", "Top/s (INT32 IMAD)")}
-# DRAM bytes (read + write) per prime of the engine kernel, from an ncu capture of this bench at 2
-# primes per launch (profiles/k_suffix_n16384_b2_sections.md), keyed by (n, M, d, prime bits); the
-# bench scales it by the primes per launch
-MEASURED_TRAFFIC_PER_PRIME = {(16384, 32768, 3, 50): (4.138317e9 + 4.254311e9) / 2}
 REF_DIR = os.path.join(ROOT, "oracle", "_ref")
 
 
@@ -103,6 +99,15 @@ def hbm_peak():
             return float(json.load(f)["hbm_gbs"]), "measured"
     except (OSError, KeyError, ValueError):
         return 6650.0, "fallback"
+
+
+def hbm_record(traffic, ms):
+    """roofline.hbm: DRAM bytes per launch of the main kernel, from an ncu capture of the kernel that ran
+    (--traffic-bytes), over its device-timed duration; null without one."""
+    if not traffic:
+        return None
+    gbs, (peak, source) = traffic / (ms * 1e-3) / 1e9, hbm_peak()
+    return {"achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak, "peak_source": source}
 
 
 def host_cores():
@@ -621,13 +626,7 @@ def main():
     ops_mm, bound, ops_unit = OPS_PER_MM[a.prime_bits]
     # the timed stream holds only this engine's launches, back to back: per-GPU algorithmic rate
     achieved = B * a.steps * algorithmic_mm(n) * ops_mm / (ms * 1e-3) / 1e12
-    per_prime = MEASURED_TRAFFIC_PER_PRIME.get((n, M, d, a.prime_bits))
-    traffic = a.traffic_bytes or (per_prime * B if per_prime else None)
-    hbm = None
-    if traffic:  # the kernel's DRAM bytes per launch (ncu) over its device-timed launch duration
-        gbs = traffic / (ms / a.steps * 1e-3) / 1e9
-        peak_gbs, which = hbm_peak()
-        hbm = {"achieved": gbs, "peak": peak_gbs, "unit": "GB/s", "frac": gbs / peak_gbs, "peak_source": which}
+    hbm = hbm_record(a.traffic_bytes, ms / a.steps)
     eng.close()  # its workspace (a wave of tables) goes back before the runs below allocate theirs
 
     def section(fn, *args, **kw):
@@ -681,7 +680,7 @@ def main():
                        "l2": "inputs larger than L2 (per-prime tables total far above 126 MB)"},
             "roofline": {"bound": bound, "achieved": achieved, "peak": peak, "unit": ops_unit,
                          "frac": achieved / peak if peak else None,
-                         "traffic": traffic, "hbm": hbm,
+                         "traffic": a.traffic_bytes, "hbm": hbm,
                          "model": f"{ops_mm} {bound} operations per modular multiplication, "
                                   f"{algorithmic_mm(n):.3e} multiplications per prime-residue; peak measured live"},
             "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches, "clocks": clk.summary(),
