@@ -95,8 +95,7 @@ static int resident_clusters(const KInfo& ki, size_t smem, cudaStream_t s) {
 }
 // The cluster geometry a launch at transform length 2^lg runs: the one pinned on the engine
 // (cf_tune_set, or cf_autotune's choice), else the default, the first of cluster_variants.
-static KInfo pick_cluster(const cf_engine* e, int lg, int nb, int J, cudaStream_t s, bool wide = false) {
-    (void)nb, (void)J, (void)s;
+static KInfo pick_cluster(const cf_engine* e, int lg, bool wide = false) {
     KInfo v[8];
     if (wide) return kernel_for(lg, true);
     const int k = cluster_variants(lg, v);
@@ -300,7 +299,7 @@ static int launch_batch(cf_engine* e, const u64* d_primes, int B, int nmax, int 
     KInfo ki = pl.ki;
     if (!ki.fn) return fail(e, CF_ERR_UNSUPPORTED, "no kernel for this transform length");
     if (ki.cluster > 1 && keep) return fail(e, CF_ERR_UNSUPPORTED, "resident tables are built up to nmax = 16384");
-    if (ki.cluster > 1) ki = pick_cluster(e, pl.lg, B, J, s, pl.wide);
+    if (ki.cluster > 1) ki = pick_cluster(e, pl.lg, pl.wide);
     size_t smem = 0;
     int JC = 0;
     int rc0 = plan_queries(e, pl.lg, ki, J, &smem, &JC);
@@ -679,7 +678,7 @@ long cf_resident_primes(cf_engine* e, int nmax, int Mmax, int J) {
     std::vector<int> qn((size_t)std::max(J, 1), nmax), qM((size_t)std::max(J, 1), std::max(Mmax, nmax + 1));
     Plan pl;
     if (plan(e, nmax, 3, CF_MODEL_SUBSET, qn.data(), qM.data(), J, pl)) return 0;
-    const KInfo ki = pl.ki.cluster > 1 ? pick_cluster(e, pl.lg, 1, J, e->stream) : pl.ki;
+    const KInfo ki = pl.ki.cluster > 1 ? pick_cluster(e, pl.lg) : pl.ki;
     size_t smem = 0;
     int JC = 0;
     if (plan_queries(e, pl.lg, ki, J, &smem, &JC)) return 0;

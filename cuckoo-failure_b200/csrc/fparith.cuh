@@ -3,9 +3,10 @@
 // A residue is a double holding a whole number x with |x| <= a p for a small bound a (values are
 // signed and not canonical; every function states its bounds in multiples of p).  The product of
 // two residues takes six double-precision operations, all of which issue at 64 per SM per clock on
-// B200, where a 64-bit Shoup product takes nine 32-bit multiplies of the same rate and about as many
-// adds: measured in registers, radix-32 passes of butterflies run at 7.0 butterflies per SM per
-// clock this way and at 3.6 .. 3.9 with integers.
+// B200 (a butterfly takes eight), where a 64-bit Shoup product takes nine 32-bit multiplies of the same
+// rate and about as many adds.  n = 16384, 148 primes: 66.6 primes a second with integers, 148 this way.
+// The product is the one of van der Hoeven, Lecerf and Quintin, "Modular SIMD arithmetic in Mathemagix"
+// (2016): the high part of x w, its error by an FMA, a rounded quotient and its remainder.
 //
 // Why it is exact (p < 2^50, |x w| <= 2^51 p):
 //   h = fl(x w); x w = h + l with l = fma(x, w, -h) exact (an FMA's rounding error of a product).
@@ -51,14 +52,9 @@ struct FpMod {
     double p, pinv;  // the prime and fl(1/p)
 };
 
-// the whole number nearest x, |x| <= 2^51
-CF_HD double fp_round(double x) {
-    constexpr double M = 6755399441055744.0;  // 1.5 2^52
-    return fp_add(fp_add(x, M), -M);
-}
 // x w mod p: |result| <= (1/2 + a b / 4) p for |x| <= a p, |w| <= b p, a b <= 2
 CF_HD double fp_mulmod(double x, double w, const FpMod& m) {
-    constexpr double M = 6755399441055744.0;
+    constexpr double M = 6755399441055744.0;  // 1.5 2^52
     const double h = fp_mul(x, w);
     const double q = fp_add(fp_fma(h, m.pinv, M), -M);
     const double l = fp_fma(x, w, -h);

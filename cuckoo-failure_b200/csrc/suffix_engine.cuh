@@ -21,7 +21,7 @@
 //     (each thread holds the entries t + k T);
 //   * the queries are evaluated on the fly from the stage-1 input rows (the same U[w] the
 //     reference's k_query builds), over the row's live entries only; each warp leaves its partial
-//     sum in shared memory and, after the transform's first barrier, one warp per query folds the
+//     sum in shared memory and, after a barrier of the transform, a thread per query folds the
 //     row's partials into one word, so a batch needs no separate pass over V and no barrier of its
 //     own per row.
 //
@@ -530,8 +530,11 @@ struct PrimeBase {
 
     // The full tile's columns v0 .. v0 + 15 into row storage, the rows r = t + jT of the warp's threads (rows of
     // later groups only: a row of this tile's group reads these columns from the tile).  The warp wrote
-    // the staged columns of these rows itself, so only its own threads need to meet before it, and the
-    // cells written were last read by an earlier step.  Four lanes take a row, four columns each, so a
+    // the staged columns of these rows itself, so only its own threads need to meet before it.  Other warps
+    // may have read the cells written: a block that the flush replaces holds rows of this tile's group, of
+    // which row v = v0 + 15 of V was read in step v - 1, and row v of S in stage 1 of this step.  So
+    // the flush must stay behind the barriers of step v's second convolution, which every thread
+    // passes after that read of S.  Four lanes take a row, four columns each, so a
     // store instruction fills eight whole 128-byte lines (one row per lane wrote a sector of 32 lines:
     // the flush was bound by those).
     CF_HD void flush_rows(int t, int v0) const {
