@@ -496,9 +496,20 @@ struct PrimeBase {
 
     // Row q's per-warp partials of queries ja .. jb - 1 (written before a barrier) into ps[j][q], a thread
     // per query.  A query with n_j < q has none: its word of row q is never read.
+    // Clusters of the integer kernels: a warp per query, with shuffles.  Their fold stands in every CTA's
+    // way to the next cluster barrier (ms a thread per query, a warp; n = 20000, 24 primes: one query 1861,
+    // 1844, nine 1991, 1971; 16 primes, 40 queries 2512, 2484; n = 40000, 4 primes: 3800, 3804).  On one CTA
+    // a warp per query is the slower form (n = 3000, 128 primes: 129.7, 131.7; n = 16384, 148: 3602, 3648).
     CF_HD void fold_queries(int q, int ja, int jb) {
         const u64* qs = sm + SM::QS;
         ex.each([&](int t, Regs<G>&) CF_INL {
+            if constexpr (K == 1 && C > 1) {
+                for (int jq = ja + (lt(t) >> 5), lane = t & 31; jq < jb; jq += NW) {
+                    const u64 v = lane < NW ? qs[(size_t)(jq - ja) * NW + lane] : 0;
+                    ex.warp_sum_store(lt(t), v, P, ps() + (size_t)jq * (kp.n + 1) + q, 0);
+                }
+                return;
+            }
             for (int jq = ja + lt(t); jq < jb; jq += CT) {
                 u64 s = 0;
 #pragma unroll 4
