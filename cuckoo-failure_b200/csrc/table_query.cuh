@@ -14,7 +14,7 @@
 // table, n = 2048, 148 primes: 2.5 GB), by the products (seven double-precision operations each) where
 // many do.  A warp reads 2 KB of a row at a time, a row ahead: with 256 bytes of four rows at a
 // time, summing along the rows, HBM gave 2.2 TB/s (1320 us for that case); the form before that, one
-// CTA of 64-bit integer products per (prime, query), took 3570 us; this one takes 610 to 700 (3.6 to 4.1 TB/s).
+// CTA of 64-bit integer products per (prime, query), took 3570 us; this one takes 600 to 700 (3.6 to 4.2 TB/s).
 #pragma once
 #include <cuda_runtime.h>
 
